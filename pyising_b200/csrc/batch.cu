@@ -97,7 +97,7 @@ static_assert(sizeof(Int8Launch) <= 32764, "kernel parameter block over the 32 K
 
 template <int V, int NDIM, int RULE, bool MIXED, bool MEAS>
 __device__ __forceinline__ void batch_int8_slots(const Int8Half& p, const Int8Desc& L, u32 s0,
-                                                 u32 s1, const u32* stab, long long& m_acc,
+                                                 u32 s1, const u32* rt, long long& m_acc,
                                                  long long& e_acc)
 {
     const u32 cpr = (u32)L.cpr, bpp = (u32)L.bpp;
@@ -111,7 +111,7 @@ __device__ __forceinline__ void batch_int8_slots(const Int8Half& p, const Int8De
         }
         const int y0 = yb * L.band;
         const int y1 = y0 + L.band < L.ly ? y0 + L.band : L.ly;
-        int8_band<V, NDIM, RULE, MIXED, MEAS>(p, z, y0, y1, j0, stab, m_acc, e_acc);
+        int8_band<V, NDIM, RULE, MIXED, MEAS>(p, z, y0, y1, j0, rt, m_acc, e_acc);
     }
 }
 
@@ -122,7 +122,7 @@ template <int V, int NDIM, int RULE, bool MIXED, int N>
 __global__ void __launch_bounds__(256, ISING_BATCH_MIN_BLOCKS)
     batch_int8_kernel(const __grid_constant__ Int8LaunchN<N> P)
 {
-    __shared__ u32 stab[8];  // acceptance table for the per-site lookup rules
+    __shared__ u32 rt[kLookupWords];  // the lookup table of the decisions
     // launched with programmatic stream serialization: wait for the previous kernel of the
     // stream (every kernel of the engine's stream waits on its predecessor in turn, so this
     // class's previous half-sweep has completed too), then let the next launch start
@@ -136,13 +136,8 @@ __global__ void __launch_bounds__(256, ISING_BATCH_MIN_BLOCKS)
         else hi = mid - 1;
     }
     const Int8Desc& L = P.lat[lo];
-    if constexpr (RULE != kMetroFast) {
-        if (threadIdx.x == 0) {
-#pragma unroll
-            for (int i = 0; i < 7; ++i) stab[i] = L.table[i];
-        }
-        __syncthreads();
-    }
+    if (threadIdx.x == 0) fill_lookup<NDIM, RULE>(rt, L.table);
+    __syncthreads();
     const long long epoch = P.epoch + (P.epoch_base ? *P.epoch_base : 0);
     const u32 color = (u32)(epoch & 1);
     const u32 s = (u32)((epoch - L.join_epoch) >> 1);  // sweeps done (< 2^31)
@@ -171,10 +166,10 @@ __global__ void __launch_bounds__(256, ISING_BATCH_MIN_BLOCKS)
     const u32 s1 = s0 + (u32)L.per_block < (u32)L.nslots ? s0 + (u32)L.per_block : (u32)L.nslots;
     long long m_acc = 0, e_acc = 0;
     if (meas) {
-        batch_int8_slots<V, NDIM, RULE, MIXED, true>(p, L, s0, s1, stab, m_acc, e_acc);
+        batch_int8_slots<V, NDIM, RULE, MIXED, true>(p, L, s0, s1, rt, m_acc, e_acc);
         block_accumulate2(m_acc, e_acc, p.meas);
     } else {
-        batch_int8_slots<V, NDIM, RULE, MIXED, false>(p, L, s0, s1, stab, m_acc, e_acc);
+        batch_int8_slots<V, NDIM, RULE, MIXED, false>(p, L, s0, s1, rt, m_acc, e_acc);
     }
 }
 
@@ -809,13 +804,10 @@ private:
         switch (rule) {
         case kMetroFast:
             return launch_pdl(batch_int8_kernel<V, NDIM, kMetroFast, MIXED, N>, grid, block, stream_, P);
-        case kHeatFast:
-            return launch_pdl(batch_int8_kernel<V, NDIM, kHeatFast, MIXED, N>, grid, block, stream_, P);
+        case kHeat:
+            return launch_pdl(batch_int8_kernel<V, NDIM, kHeat, MIXED, N>, grid, block, stream_, P);
         case kMetroGeneric:
             return launch_pdl(batch_int8_kernel<V, NDIM, kMetroGeneric, MIXED, N>, grid, block,
-                              stream_, P);
-        case kHeatGeneric:
-            return launch_pdl(batch_int8_kernel<V, NDIM, kHeatGeneric, MIXED, N>, grid, block,
                               stream_, P);
         default: return cudaErrorInvalidValue;
         }

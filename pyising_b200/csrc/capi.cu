@@ -114,14 +114,12 @@ int select_rule(int variant, int algorithm, int ndim, const u32* table)
     if (variant == ISING_VARIANT_MSC) return kMetroFast;
     const int d = ndim;
     if (algorithm == ISING_METROPOLIS) {
-        // the fast rule needs T(a) = table[2d - a] non-decreasing in a < d
-        for (int i = d + 1; i < 2 * d; ++i)
-            if (table[i] < table[i + 1]) return kMetroGeneric;
+        // the fast rule holds the largest flipping uniform of each count: there must be one
+        for (int i = d + 1; i <= 2 * d; ++i)
+            if (table[i] == 0) return kMetroGeneric;
         return kMetroFast;
     }
-    for (int i = 0; i < 2 * d; ++i)
-        if (table[i] > table[i + 1]) return kHeatGeneric;
-    return kHeatFast;
+    return kHeat;
 }
 
 }  // namespace ising

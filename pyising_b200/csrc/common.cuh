@@ -6,6 +6,7 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 #include <utility>
 
 #include <cuda_runtime.h>
@@ -60,13 +61,11 @@ __device__ __forceinline__ u32x4 philox4x32_10(u32 c0, u32 c1, u32 c2, u32 c3, u
     return u32x4{c0, c1, c2, c3};
 }
 
-// Byte lanes of packed int8 spins: +1 is 0x01, -1 is 0xFF, so bit 1 of a byte is the
-// "spin down" flag and (a ^ b) & 0x02 is the "anti-aligned" flag of two spins.
-constexpr u32 kBit1 = 0x02020202u;
-constexpr u32 kBit7 = 0x80808080u;
-
-// 0x80 per selected byte -> 0xFE per selected byte (the XOR that flips a +-1 byte).
-__device__ __forceinline__ u32 flip_mask_from_bit7(u32 m7) { return m7 | (m7 - (m7 >> 6)); }
+// Byte lanes of packed int8 spins: +1 is 0x01, -1 is 0xFF, so bits 1 to 7 of a byte are the
+// "spin down" flag, and XOR with 0xFE flips.
+constexpr u32 kBit2 = 0x04040404u;
+constexpr u32 kBit5 = 0x20202020u;
+constexpr u32 kFlip = 0xFEFEFEFEu;
 
 // Sum of the four bytes of v (each byte small and non-negative).
 __device__ __forceinline__ int byte_sum(u32 v) { return (int)__dp4a(v, 0x01010101u, 0u); }
@@ -110,11 +109,9 @@ __device__ __forceinline__ void block_accumulate2(long long a, long long b,
 
 // Decision rule selected on the host.
 enum Rule : int {
-    kMetroFast = 0,    // Metropolis, table[d+1..2d] non-increasing (always true for tables
-                       // built by threshold_table)
-    kHeatFast = 1,     // heat bath, table non-decreasing (beta >= 0)
-    kMetroGeneric = 2, // any table, one lookup per site
-    kHeatGeneric = 3,
+    kMetroFast = 0,    // Metropolis, table[d+1..2d] without a zero (2D: beta < 2.77)
+    kHeat = 1,         // heat bath
+    kMetroGeneric = 2, // Metropolis, any table
     kObserve = 4,      // no update: measurement only
 };
 

@@ -8,15 +8,18 @@
 //
 // Work split: a thread owns V consecutive colour sites of one row (V = 16: one 128-bit load
 // per array, four Philox blocks).  Spins stay packed in 32-bit words and the neighbour
-// counting is byte-parallel (SWAR): with +1 = 0x01 and -1 = 0xFF, bit 1 of each byte is the
-// "down" flag, so (a ^ b) & 0x02020202 marks anti-aligned pairs of four sites at once.
+// counting is byte-parallel (SWAR): with +1 = 0x01 and -1 = 0xFF, bits 1 to 7 of a byte are the
+// "down" flag.  A loaded word of the opposite colour is masked once with 0x04040404, so the sum
+// of a site's neighbour words holds four times its down neighbours D: the byte offset of an
+// entry in a table of 32-bit thresholds.
 //
-// Metropolis decision without lookups.  Metropolis flips iff X <= 0 or u < table[(X + 2d)/2]
-// with X = s*h = 2d - 2A (A = anti-aligned neighbours).  Let T(a) = table[2d - a] for a < d;
-// threshold tables built by threshold_table() make T non-decreasing in a, so with
-// L = #{a < d : u < T(a)} the rule is exactly "flip iff A + L >= d", evaluated byte-parallel.
-// Heat bath (+1 iff u < table[U], U = up neighbours = 2d - D) and Metropolis with a table that
-// is not monotone read table[.] per site from a shared-memory copy of the table.
+// Decision: one shared-memory lookup, one comparison and one predicated operation per site.
+//   Heat bath: +1 iff u < table[U], U = up neighbours = 2d - D.
+//   Metropolis flips iff X <= 0 or u < table[(X + 2d)/2], X = s*h = 2d - 2A, A = anti-aligned
+//   neighbours = D for an up spin, 2d - D for a down spin.  The lookup index is 4 D + 32 (spin
+//   down), the entry the largest uniform that flips: table[2d - A] - 1 for A < d, 2^32 - 1 (every
+//   uniform) for A >= d.  A table with a zero among its A < d entries (no uniform flips) has no
+//   such entry and takes the general rule.
 #pragma once
 
 #include "common.cuh"
@@ -97,168 +100,191 @@ __device__ __forceinline__ void store_words(int8_t* p, const Words<W>& r)
     }
 }
 
-// 32-bit load from a shared-memory byte address.
-__device__ __forceinline__ u32 lds_u32(u32 addr)
+// Words of the opposite colour as the neighbour sums take them: 4 for a down spin, 0 for up.
+template <int W>
+__device__ __forceinline__ Words<W> downs(Words<W> w)
 {
-    u32 v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-    return v;
+#pragma unroll
+    for (int k = 0; k < W; ++k) w.v[k] &= kBit2;
+    return w;
 }
 
-// 4-bit mask (bit i = site i) -> XOR pattern 0xFE in byte i (the flip of a +-1 byte).
-__device__ __forceinline__ u32 flip_bytes(u32 m4)
-{
-    return ((m4 * 0x00204081u) & 0x01010101u) * 0xFEu;  // bit i -> byte i, then 0x01 -> 0xFE
-}
+// The lookup table of a block (kLookupWords words of shared memory), indexed by the byte offset
+// 4 D (heat bath; also the general Metropolis rule's thresholds) or 4 D + 32 (own spin down).
+// Padding bytes hold any value, so every offset that their masked sums can form is in range:
+// 4 * 6 + 32 bytes at most.  One thread fills it.
+constexpr int kLookupWords = 16;
 
-// New spins of the four sites in word `s` given their anti-aligned (Metropolis) or down
-// (heat bath) neighbour counts `cnt` (one byte per site) and their four uniforms.  `stab` is
-// the acceptance table in shared memory (used by the lookup rules).
-//   kMetroFast: byte-parallel "A + #{a<d : u < T(a)} >= d" (monotone Metropolis tables);
-//   heat bath and kMetroGeneric: one shared-memory lookup per site, valid for any table.
 template <int NDIM, int RULE>
-__device__ __forceinline__ u32 decide4(const Int8Half& p, u32 s, u32 cnt, const u32x4& r,
-                                       const u32* stab)
+__device__ __forceinline__ void fill_lookup(u32* rt, const u32* table)
 {
     constexpr int d = NDIM;
-    if constexpr (RULE == kObserve) {
-        return s;
-    } else if constexpr (RULE == kMetroFast) {
-        u32 l[4] = {0, 0, 0, 0};
-        const u32 uu[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
-        for (int a = 0; a < d; ++a) {
-            const u32 thr = p.table[2 * d - a];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) l[i] += uu[i] < thr ? 1u : 0u;
+    for (int i = 0; i < kLookupWords; ++i) {
+        const int D = i & 7, a = i < 8 ? D : 2 * d - D;  // a: anti-aligned neighbours
+        if (D > 2 * d) {
+            rt[i] = 0u;
+        } else if constexpr (RULE == kHeat) {
+            rt[i] = table[2 * d - D];
+        } else if constexpr (RULE == kMetroFast) {
+            rt[i] = a < d ? table[2 * d - a] - 1u : 0xFFFFFFFFu;
+        } else {
+            rt[i] = a < d ? table[2 * d - a] : 0u;
         }
-        const u32 lw = l[0] | (l[1] << 8) | (l[2] << 16) | (l[3] << 24);
-        const u32 m7 = (cnt + lw + (u32)(0x80 - d) * 0x01010101u) & kBit7;
-        return s ^ flip_mask_from_bit7(m7);
-    } else if constexpr (RULE == kHeatFast || RULE == kHeatGeneric) {
-        // +1 iff u < table[U], U = up neighbours = 2d - D; rt[k] = table[2d - k]
-        const u32 base = (u32)__cvta_generic_to_shared(stab) + 8u * d;  // &table[2d]
-        const u32 b0 = r.x < lds_u32(base - 4u * (cnt & 0xFFu)) ? 1u : 0u;
-        const u32 b1 = r.y < lds_u32(base - 4u * ((cnt >> 8) & 0xFFu)) ? 2u : 0u;
-        const u32 b2 = r.z < lds_u32(base - 4u * ((cnt >> 16) & 0xFFu)) ? 4u : 0u;
-        const u32 b3 = r.w < lds_u32(base - 4u * (cnt >> 24)) ? 8u : 0u;
-        return 0xFFFFFFFFu ^ flip_bytes(b0 | b1 | b2 | b3);
-    } else {
-        // Metropolis, any table: flip iff A >= d or u < table[2d - A]
-        const u32 base = (u32)__cvta_generic_to_shared(stab) + 8u * d;  // &table[2d]
-        const u32 a0 = cnt & 0xFFu, a1 = (cnt >> 8) & 0xFFu, a2 = (cnt >> 16) & 0xFFu,
-                  a3 = cnt >> 24;
-        const u32 f0 = (a0 >= (u32)d || r.x < lds_u32(base - 4u * a0)) ? 1u : 0u;
-        const u32 f1 = (a1 >= (u32)d || r.y < lds_u32(base - 4u * a1)) ? 2u : 0u;
-        const u32 f2 = (a2 >= (u32)d || r.z < lds_u32(base - 4u * a2)) ? 4u : 0u;
-        const u32 f3 = (a3 >= (u32)d || r.w < lds_u32(base - 4u * a3)) ? 8u : 0u;
-        return s ^ flip_bytes(f0 | f1 | f2 | f3);
     }
 }
 
-// New spins of the V colour sites starting at j0 in row `row` (parity `par` = (y + z + colour)
-// & 1) from their own words `s`, the opposite colour's words of the same row `c`, of the rows
-// above/below `nu`/`nd` and planes above/below `zu`/`zd` (3D), and the horizontal neighbour byte
-// outside the chunk `edge`; stores them, and with MEAS adds the chunk's (M, E) contribution to
-// m_acc / e_acc.  With RULE == kObserve nothing is updated (measurement only).
+__device__ __forceinline__ u32 lookup(const u32* rt, u32 idx, int i)
+{
+    // byte i of idx, as a dot product: that runs on the multiplier pipe, a permute or shift on
+    // the logic pipe, which bounds the kernel
+    const u32 off = __dp4a(idx, 1u << (8 * i), 0u);
+    return *reinterpret_cast<const u32*>(reinterpret_cast<const char*>(rt) + off);
+}
+
+// Predicated operations on one byte of a word of four spins: a comparison and the operation
+// itself.  (The compiler's own form of such selects was a comparison, a conditional move and a
+// select or add per site; its moves ran on the multiplier pipe that the Philox products need.)
+__device__ __forceinline__ void add_if_less(u32& w, u32 u, u32 thr, u32 x)
+{
+    asm("{\n\t.reg .pred p;\n\tsetp.lt.u32 p, %1, %2;\n\t@p add.u32 %0, %0, %3;\n\t}"
+        : "+r"(w)
+        : "r"(u), "r"(thr), "r"(x));
+}
+
+__device__ __forceinline__ void add_if_not_greater(u32& w, u32 u, u32 thr, u32 x)
+{
+    asm("{\n\t.reg .pred p;\n\tsetp.le.u32 p, %1, %2;\n\t@p add.u32 %0, %0, %3;\n\t}"
+        : "+r"(w)
+        : "r"(u), "r"(thr), "r"(x));
+}
+
+// Bit 7 of each byte, over the whole byte (prmt's sign mode, which __byte_perm does not have).
+__device__ __forceinline__ u32 byte_signs(u32 v)
+{
+    u32 r;
+    asm("prmt.b32 %0, %1, 0, 0xBA98;" : "=r"(r) : "r"(v));
+    return r;
+}
+
+// New spins of the four sites in word `s` given four times their down neighbours `d4` (one byte
+// per site) and their four uniforms; `rt` is the block's lookup table (fill_lookup).
+template <int NDIM, int RULE>
+__device__ __forceinline__ u32 decide4(u32 s, u32 d4, const u32x4& r, const u32* rt)
+{
+    constexpr int d = NDIM;
+    const u32 u[4] = {r.x, r.y, r.z, r.w};
+    if constexpr (RULE == kObserve) {
+        return s;
+    } else if constexpr (RULE == kHeat) {
+        u32 ns = 0xFFFFFFFFu;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) add_if_less(ns, u[i], lookup(rt, d4, i), 0u - (0xFEu << (8 * i)));
+        return ns;
+    } else if constexpr (RULE == kMetroFast) {
+        const u32 idx = d4 + (s & kBit5);
+        u32 flips = 0u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) add_if_not_greater(flips, u[i], lookup(rt, idx, i), 1u << (8 * i));
+        return s ^ (flips * 0xFEu);
+    } else {
+        // any table: A >= d flips whatever the uniform (the lookup holds 0 there)
+        const u32 idx = d4 + (s & kBit5);
+        const u32 up = d4 + (u32)(0x80 - 4 * d) * 0x01010101u;  // bit 7: D >= d
+        const u32 dn = (u32)(0x80 + 4 * d) * 0x01010101u - d4;  // bit 7: D <= d
+        u32 flips = (((up & ~s) | (dn & s)) >> 7) & 0x01010101u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) add_if_less(flips, u[i], lookup(rt, idx, i), 1u << (8 * i));
+        return s ^ (flips * 0xFEu);
+    }
+}
+
+// New spins of V consecutive colour sites of a row (parity `par` = (y + z + colour) & 1) from their
+// own words `s` and the masked words (downs) of the opposite colour: the same row
+// `c`, the rows above/below `nu`/`nd`, the planes above/below `zu`/`zd` (3D) and the horizontal
+// neighbour byte outside the chunk `edge` (masked too); with MEAS adds the chunk's (M, E)
+// contribution to m_acc / e_acc.  With RULE == kObserve nothing is updated (measurement only).
+// `draw(k)` returns the four uniforms of the chunk's word k.
 //
 // MIXED = false: every chunk is full (lh % V == 0).  MIXED = true: rows are padded to a multiple
 // of V bytes and a row's last chunk holds wv < W valid words; such a chunk runs the same
 // instructions as a full one (no divergence inside a warp), with the padding words selected
 // away: their random numbers are drawn and discarded, their bytes stored back unchanged, and
 // the right-hand neighbour of the last valid word is the row's wrapped edge byte.
-// Returns the new words; STORE = false leaves storing them to the caller (the tiles of the
-// temporally blocked kernel live in shared memory).
-template <int V, int NDIM, int RULE, bool MIXED, bool MEAS, bool STORE = true>
-__device__ __forceinline__ Words<V / 4> int8_update(const Int8Half& p, long long row, int par,
-                                                    int j0, int wv, const Words<V / 4>& s,
+template <int V, int NDIM, int RULE, bool MIXED, bool MEAS, class Draw>
+__device__ __forceinline__ Words<V / 4> int8_update(const Draw& draw, int par, int wv,
+                                                    const Words<V / 4>& s,
                                                     const Words<V / 4>& c,
                                                     const Words<V / 4>& nu,
                                                     const Words<V / 4>& nd,
                                                     const Words<V / 4>& zu,
                                                     const Words<V / 4>& zd, u32 edge,
-                                                    const u32* stab, long long& m_acc,
+                                                    const u32* rt, long long& m_acc,
                                                     long long& e_acc)
 {
     constexpr int W = V / 4;
-    constexpr bool kHeat = (RULE == kHeatFast || RULE == kHeatGeneric);
-    Words<W> hz;
-#pragma unroll
-    for (int k = 0; k < W; ++k) {
-        if (par) {
-            u32 nx = edge;
-            if (k + 1 < W) nx = (!MIXED || k + 1 < wv) ? c.v[k + 1] : edge;
-            hz.v[k] = __funnelshift_r(c.v[k], nx, 8);
-        } else {
-            const u32 pv = (k > 0) ? c.v[k - 1] : (edge << 24);
-            hz.v[k] = __funnelshift_l(pv, c.v[k], 8);
-        }
-    }
-
-    // Neighbour counts first, so the neighbour words are dead before the Philox blocks.
-    u32 cnt[W];
+    // Neighbour sums first, so the neighbour words are dead before the Philox blocks.
+    u32 d4[W];
     int other_down = 0;  // down spins of the opposite colour at the same indices (for M)
 #pragma unroll
     for (int k = 0; k < W; ++k) {
-        if constexpr (kHeat) {
-            u32 acc = (c.v[k] & kBit1) + (hz.v[k] & kBit1) + (nu.v[k] & kBit1) +
-                      (nd.v[k] & kBit1);
-            if constexpr (NDIM == 3) acc += (zu.v[k] & kBit1) + (zd.v[k] & kBit1);
-            cnt[k] = acc >> 1;  // down neighbours per site
+        u32 hz;  // the horizontal neighbours that are not at the sites' own indices
+        if (par) {
+            u32 nx = edge;
+            if (k + 1 < W) nx = (!MIXED || k + 1 < wv) ? c.v[k + 1] : edge;
+            hz = __byte_perm(c.v[k], nx, 0x4321);
         } else {
-            const u32 sv = s.v[k];
-            u32 acc = ((c.v[k] ^ sv) & kBit1) + ((hz.v[k] ^ sv) & kBit1) +
-                      ((nu.v[k] ^ sv) & kBit1) + ((nd.v[k] ^ sv) & kBit1);
-            if constexpr (NDIM == 3)
-                acc += ((zu.v[k] ^ sv) & kBit1) + ((zd.v[k] ^ sv) & kBit1);
-            cnt[k] = acc >> 1;  // anti-aligned neighbours per site
+            hz = k > 0 ? __byte_perm(c.v[k], c.v[k - 1], 0x2107) : __byte_perm(c.v[k], edge, 0x2104);
         }
+        d4[k] = c.v[k] + nu.v[k] + nd.v[k] + hz;
+        if constexpr (NDIM == 3) d4[k] += zu.v[k] + zd.v[k];
         if constexpr (MEAS) {
-            const int od = __popc(c.v[k] & kBit1);
+            const int od = __popc(c.v[k]);
             other_down += (!MIXED || k < wv) ? od : 0;
         }
     }
 
     Words<W> ns;
-    // Philox counters use the logical site index row*lh + j, independent of the pitch
-    const u32 q0 = (u32)((unsigned long long)(row * p.lh + j0) >> 2);
 #pragma unroll
     for (int k = 0; k < W; ++k) {
         if constexpr (RULE == kObserve) {
             ns.v[k] = s.v[k];
         } else {
-            const u32x4 r =
-                philox4x32_10<NDIM == 2>(q0 + (u32)k, p.t, p.color, 0u, p.k0, p.k1);
-            const u32 d = decide4<NDIM, RULE>(p, s.v[k], cnt[k], r, stab);
+            const u32 d = decide4<NDIM, RULE>(s.v[k], d4[k], draw(k), rt);
             ns.v[k] = (!MIXED || k < wv) ? d : s.v[k];
         }
     }
-    if constexpr (RULE != kObserve && STORE) store_words<W>(p.own + row * p.pitch + j0, ns);
 
     if constexpr (MEAS) {
-        // Bonds of this colour's sites: s*h = 2d - 2A' per site (A' = anti-aligned neighbours
-        // of the new spin); E = -sum s*h.  A' follows from the counts: a flipped site's
-        // anti-aligned neighbours are the previously aligned ones (2d - A), and for heat bath
-        // A' = D for a +1 site, 2d - D for a -1 site.
-        constexpr u32 k2d = 0x01010101u * (u32)(2 * NDIM);
-        int anti = 0, down = 0;
+        // Bonds of this colour's sites: s*h = 2d - 2A' per site, A' = anti-aligned neighbours of
+        // the new spin: D if it is up, 2d - D if it is down; E = -sum s*h.
+        constexpr u32 k8d = 0x01010101u * (u32)(8 * NDIM);
+        int anti4 = 0, down = 0;
 #pragma unroll
         for (int k = 0; k < W; ++k) {
-            const u32 sv = ns.v[k];
-            u32 sel;  // 0xFF in the bytes whose count is replaced by 2d - count
-            if constexpr (kHeat) sel = ((sv & kBit1) >> 1) * 0xFFu;
-            else sel = (((sv ^ s.v[k]) & kBit1) >> 1) * 0xFFu;
-            const u32 ap = (cnt[k] & ~sel) | ((k2d - cnt[k]) & sel);
+            const u32 sel = byte_signs(ns.v[k]);
+            const u32 a4 = (d4[k] & ~sel) | ((k8d - d4[k]) & sel);
             const bool valid = !MIXED || k < wv;
-            anti += valid ? byte_sum(ap) : 0;
-            down += valid ? __popc(sv & kBit1) : 0;
+            anti4 += valid ? byte_sum(a4) : 0;
+            down += valid ? __popc(ns.v[k] & kBit2) : 0;
         }
         const int nv = 4 * wv;                      // valid sites of this chunk
         m_acc += 2 * nv - 2 * (down + other_down);  // this colour's sites + the other's
-        e_acc += 2 * anti - 2 * NDIM * nv;          // -(2d n - 2 anti)
+        e_acc += anti4 / 2 - 2 * NDIM * nv;         // -(2d n - 2 anti)
     }
     return ns;
 }
+
+// The four uniforms of word k of the chunk whose first four sites have Philox counter q0.
+template <int NDIM>
+struct DrawSites {
+    const Int8Half& p;
+    u32 q0;
+    __device__ __forceinline__ u32x4 operator()(int k) const
+    {
+        return philox4x32_10<NDIM == 2>(q0 + (u32)k, p.t, p.color, 0u, p.k0, p.k1);
+    }
+};
 
 template <bool MIXED, int W>
 __device__ __forceinline__ int valid_words(const Int8Half& p, int j0)
@@ -274,11 +300,19 @@ __device__ __forceinline__ int edge_index(const Int8Half& p, int par, int j0, in
     return par ? (j0 + 4 * wv == p.lh ? 0 : j0 + 4 * wv) : (j0 == 0 ? p.lh - 1 : j0 - 1);
 }
 
+// Philox counter of the four sites from j0 of row `row`: the logical site index row*lh + j over
+// 4, independent of the pitch.
+__device__ __forceinline__ u32 site_counter(const Int8Half& p, long long row, int j0)
+{
+    return (u32)((unsigned long long)(row * p.lh + j0) >> 2);
+}
+
 // One chunk (V sites from j0) of row `row` = (z, y): loads its neighbourhood, then int8_update.
 // CG reads the opposite colour from L2 (needed when one launch runs several half-sweeps).
-template <int V, int NDIM, int RULE, bool CG, bool MIXED, bool MEAS>
-__device__ __forceinline__ void int8_chunk(const Int8Half& p, long long row, int y, int z, int j0,
-                                           const u32* stab, long long& m_acc, long long& e_acc)
+template <int V, int NDIM, int RULE, bool CG, bool MIXED, bool MEAS, class Draw>
+__device__ __forceinline__ void int8_chunk(const Int8Half& p, const Draw& draw, long long row,
+                                           int y, int z, int j0, const u32* rt, long long& m_acc,
+                                           long long& e_acc)
 {
     constexpr int W = V / 4;
     const int par = (y + z + (int)p.color) & 1;
@@ -286,53 +320,120 @@ __device__ __forceinline__ void int8_chunk(const Int8Half& p, long long row, int
     const long long rb = row * p.pitch;
     const int8_t* orow = p.other + rb;
     const Words<W> s = load_words<W>(p.own + rb + j0);
-    const Words<W> c = load_other<W, CG>(orow + j0);
+    const Words<W> c = downs(load_other<W, CG>(orow + j0));
     const int yu = z * p.ly + (y + 1 == p.ly ? 0 : y + 1);
     const int yd = z * p.ly + (y == 0 ? p.ly - 1 : y - 1);
-    const Words<W> nu = load_other<W, CG>(p.other + (long long)yu * p.pitch + j0);
-    const Words<W> nd = load_other<W, CG>(p.other + (long long)yd * p.pitch + j0);
+    const Words<W> nu = downs(load_other<W, CG>(p.other + (long long)yu * p.pitch + j0));
+    const Words<W> nd = downs(load_other<W, CG>(p.other + (long long)yd * p.pitch + j0));
     Words<W> zu = nu, zd = nd;
     if constexpr (NDIM == 3) {
         const int pu = (z + 1 == p.lz ? 0 : z + 1) * p.ly + y;
         const int pd = (z == 0 ? p.lz - 1 : z - 1) * p.ly + y;
-        zu = load_other<W, CG>(p.other + (long long)pu * p.pitch + j0);
-        zd = load_other<W, CG>(p.other + (long long)pd * p.pitch + j0);
+        zu = downs(load_other<W, CG>(p.other + (long long)pu * p.pitch + j0));
+        zd = downs(load_other<W, CG>(p.other + (long long)pd * p.pitch + j0));
     }
     const int je = edge_index(p, par, j0, wv);
-    const u32 edge = CG ? (u32)(uint8_t)__ldcg(orow + je) : (u32)(uint8_t)__ldg(orow + je);
-    int8_update<V, NDIM, RULE, MIXED, MEAS>(p, row, par, j0, wv, s, c, nu, nd, zu, zd, edge, stab,
-                                            m_acc, e_acc);
+    const u32 edge =
+        (CG ? (u32)(uint8_t)__ldcg(orow + je) : (u32)(uint8_t)__ldg(orow + je)) & kBit2;
+    const Words<W> ns = int8_update<V, NDIM, RULE, MIXED, MEAS>(
+        draw, par, wv, s, c, nu, nd, zu, zd, edge, rt, m_acc, e_acc);
+    if constexpr (RULE != kObserve) store_words<W>(p.own + rb + j0, ns);
+}
+
+// Where a band walk is: the row's own words, the row itself and its neighbour planes in the
+// opposite colour.
+struct BandRow {
+    int8_t* own;
+    const int8_t* c;
+    const int8_t* zu;
+    const int8_t* zd;
+    u32 q;  // Philox counter of the chunk's first four sites in this row
+};
+
+// One row of a band, of parity `par`: the masked rows nd, c and nu are at hand.
+template <int V, int NDIM, int RULE, bool MIXED, bool MEAS>
+__device__ __forceinline__ void int8_band_row(const Int8Half& p, const BandRow& b, int par, int wv,
+                                              int step_l, int step_r, const Words<V / 4>& c,
+                                              const Words<V / 4>& nu, const Words<V / 4>& nd,
+                                              const u32* rt, long long& m_acc, long long& e_acc)
+{
+    constexpr int W = V / 4;
+    Words<W> zu = nu, zd = nd;
+    if constexpr (NDIM == 3) {
+        zu = downs(load_words_ro<W>(b.zu));
+        zd = downs(load_words_ro<W>(b.zd));
+    }
+    const u32 edge = (u32)(uint8_t)__ldg(b.c + (par ? step_r : step_l)) & kBit2;
+    const Words<W> s = load_words<W>(b.own);
+    const Words<W> ns = int8_update<V, NDIM, RULE, MIXED, MEAS>(
+        DrawSites<NDIM>{p, b.q}, par, wv, s, c, nu, nd, zu, zd, edge, rt, m_acc, e_acc);
+    if constexpr (RULE != kObserve) store_words<W>(b.own, ns);
 }
 
 // Band schedule: chunk column j0 of rows y0 .. y1-1 of plane z, top to bottom.  The three
-// opposite-colour rows a row needs (y-1, y, y+1) slide down the band, so each row loads one new
-// opposite-colour row (plus the planes z +- 1 in 3D) instead of three.
+// opposite-colour rows a row needs (y-1, y, y+1) slide down the band, so each row loads and masks
+// one new opposite-colour row (plus the planes z +- 1 in 3D) instead of three.  A band of an even
+// number of rows takes two rows per step: the row parity, which side the horizontal neighbours
+// are on, is then fixed in the code, and the sliding rows are renamed every second row only.
 template <int V, int NDIM, int RULE, bool MIXED, bool MEAS>
 __device__ __forceinline__ void int8_band(const Int8Half& p, int z, int y0, int y1, int j0,
-                                          const u32* stab, long long& m_acc, long long& e_acc)
+                                          const u32* rt, long long& m_acc, long long& e_acc)
 {
     constexpr int W = V / 4;
     const int wv = valid_words<MIXED, W>(p, j0);
-    const int ly = p.ly;
-    const long long plane = (long long)z * ly;
-    const int8_t* oth = p.other + j0;
-    Words<W> nd = load_words_ro<W>(oth + (plane + (y0 == 0 ? ly - 1 : y0 - 1)) * p.pitch);
-    Words<W> c = load_words_ro<W>(oth + (plane + y0) * p.pitch);
-    const long long zup = NDIM == 3 ? (long long)(z + 1 == p.lz ? 0 : z + 1) * ly : 0;
-    const long long zdn = NDIM == 3 ? (long long)(z == 0 ? p.lz - 1 : z - 1) * ly : 0;
-    for (int y = y0; y < y1; ++y) {
-        const long long row = plane + y;
-        const Words<W> nu = load_words_ro<W>(oth + (plane + (y + 1 == ly ? 0 : y + 1)) * p.pitch);
-        Words<W> zu = nu, zd = nd;
+    const int ly = p.ly, pitch = p.pitch;
+    const u32 qstep = (u32)p.lh >> 2;
+    const long long row0 = (long long)z * ly + y0;
+    const int8_t* plane = p.other + (long long)z * ly * pitch + j0;  // row 0 of the plane
+    const int step_r = j0 + 4 * wv == p.lh ? -j0 : 4 * wv, step_l = j0 == 0 ? p.lh - 1 : -1;
+    BandRow b;
+    b.own = p.own + row0 * pitch + j0;
+    b.c = plane + (long long)y0 * pitch;
+    b.q = site_counter(p, row0, j0);
+    b.zu = b.zd = b.c;
+    if constexpr (NDIM == 3) {
+        b.zu = p.other + ((long long)(z + 1 == p.lz ? 0 : z + 1) * ly + y0) * pitch + j0;
+        b.zd = p.other + ((long long)(z == 0 ? p.lz - 1 : z - 1) * ly + y0) * pitch + j0;
+    }
+    auto advance = [&] {
+        b.own += pitch;
+        b.c += pitch;
+        b.q += qstep;
         if constexpr (NDIM == 3) {
-            zu = load_words_ro<W>(oth + (zup + y) * p.pitch);
-            zd = load_words_ro<W>(oth + (zdn + y) * p.pitch);
+            b.zu += pitch;
+            b.zd += pitch;
         }
-        const int par = (y + z + (int)p.color) & 1;
-        const u32 edge = (u32)(uint8_t)__ldg(p.other + row * p.pitch + edge_index(p, par, j0, wv));
-        const Words<W> s = load_words<W>(p.own + row * p.pitch + j0);
-        int8_update<V, NDIM, RULE, MIXED, MEAS>(p, row, par, j0, wv, s, c, nu, nd, zu, zd, edge,
-                                                stab, m_acc, e_acc);
+    };
+    Words<W> nd = downs(load_words_ro<W>(y0 == 0 ? plane + (long long)(ly - 1) * pitch : b.c - pitch));
+    Words<W> c = downs(load_words_ro<W>(b.c));
+    const int par0 = (y0 + z + (int)p.color) & 1;
+    auto pairs = [&](auto par) {
+        constexpr int P = decltype(par)::value;
+#pragma unroll 1
+        for (int y = y0; y < y1; y += 2) {
+            const Words<W> d1 = downs(load_words_ro<W>(b.c + pitch));  // y is even: y + 1 < ly
+            int8_band_row<V, NDIM, RULE, MIXED, MEAS>(p, b, P, wv, step_l, step_r, c, d1, nd, rt,
+                                                      m_acc, e_acc);
+            advance();
+            const Words<W> d2 = downs(load_words_ro<W>(y + 2 == ly ? plane : b.c + pitch));
+            int8_band_row<V, NDIM, RULE, MIXED, MEAS>(p, b, 1 - P, wv, step_l, step_r, d1, d2, c,
+                                                      rt, m_acc, e_acc);
+            advance();
+            nd = d1;
+            c = d2;
+        }
+    };
+    if (((y0 | y1) & 1) == 0) {
+        if (par0) pairs(std::integral_constant<int, 1>{});
+        else pairs(std::integral_constant<int, 0>{});
+        return;
+    }
+#pragma unroll 1
+    for (int y = y0; y < y1; ++y) {
+        const Words<W> nu = downs(load_words_ro<W>(y + 1 == ly ? plane : b.c + pitch));
+        int8_band_row<V, NDIM, RULE, MIXED, MEAS>(p, b, (par0 + y - y0) & 1, wv, step_l, step_r, c,
+                                                  nu, nd, rt, m_acc, e_acc);
+        advance();
         nd = c;
         c = nu;
     }

@@ -76,13 +76,10 @@ __global__ void wait_selftest_kernel(unsigned int* flags, int* err, unsigned lon
 template <int RULE>
 __global__ void __launch_bounds__(256) int8_persistent_kernel(const PersistArgs a)
 {
-    __shared__ u32 stab[8];
+    __shared__ u32 rt[kLookupWords];  // the lookup table of the decisions
     __shared__ int s_abort;
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int i = 0; i < 7; ++i) stab[i] = a.p.table[i];
-        s_abort = 0;
-    }
+    if (threadIdx.x == 0) fill_lookup<2, RULE>(rt, a.p.table);
+    if (threadIdx.x == 0) s_abort = 0;
     __syncthreads();
     const int nb = gridDim.x, b = blockIdx.x;
     const int up = (b + nb - 1) % nb, dn = (b + 1) % nb;
@@ -113,11 +110,13 @@ __global__ void __launch_bounds__(256) int8_persistent_kernel(const PersistArgs 
         for (long long row = r0 + ty; row < r1; row += by)
             for (int jc = tx; jc < p.cpr; jc += bx) {
                 if (meas)
-                    int8_chunk<16, 2, RULE, true, true, true>(p, row, (int)row, 0, jc * 16, stab,
-                                                              m_acc, e_acc);
+                    int8_chunk<16, 2, RULE, true, true, true>(
+                        p, DrawSites<2>{p, site_counter(p, row, jc * 16)}, row, (int)row, 0, jc * 16,
+                        rt, m_acc, e_acc);
                 else
-                    int8_chunk<16, 2, RULE, true, true, false>(p, row, (int)row, 0, jc * 16, stab,
-                                                               m_acc, e_acc);
+                    int8_chunk<16, 2, RULE, true, true, false>(
+                        p, DrawSites<2>{p, site_counter(p, row, jc * 16)}, row, (int)row, 0, jc * 16,
+                        rt, m_acc, e_acc);
             }
         if (meas) block_accumulate2(m_acc, e_acc, p.meas);
         __syncthreads();  // every row of the band is written (CTA scope) ...
@@ -168,9 +167,8 @@ int run_persistent_int8(ising_sim* h, uint64_t t0, int64_t n_sweeps, int64_t mea
     const void* fn;
     switch (h->rule) {
     case kMetroFast: fn = (const void*)int8_persistent_kernel<kMetroFast>; break;
-    case kHeatFast: fn = (const void*)int8_persistent_kernel<kHeatFast>; break;
-    case kMetroGeneric: fn = (const void*)int8_persistent_kernel<kMetroGeneric>; break;
-    default: fn = (const void*)int8_persistent_kernel<kHeatGeneric>; break;
+    case kHeat: fn = (const void*)int8_persistent_kernel<kHeat>; break;
+    default: fn = (const void*)int8_persistent_kernel<kMetroGeneric>; break;
     }
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0) != cudaSuccess ||

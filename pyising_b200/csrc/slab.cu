@@ -82,11 +82,8 @@ __global__ void __launch_bounds__(256, 4) int8_slab_kernel(const Int8Half p_in, 
 {
     constexpr int V = 16, W = 4;
     Int8Half p = p_in;
-    __shared__ u32 stab[8];
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int i = 0; i < 7; ++i) stab[i] = p.table[i];
-    }
+    __shared__ u32 rt[kLookupWords];  // the lookup table of the decisions
+    if (threadIdx.x == 0) fill_lookup<NDIM, RULE>(rt, p.table);
     pdl_wait();  // the previous kernel of the stream has completed
     pdl_trigger();
     __syncthreads();
@@ -120,23 +117,24 @@ __global__ void __launch_bounds__(256, 4) int8_slab_kernel(const Int8Half p_in, 
         };
         // 2D: y is the slab axis, rows -1 and ly are halo rows; 3D: y wraps inside its plane
         const long long yprev = NDIM == 2 ? y0 - 1 : (y0 == 0 ? ly - 1 : y0 - 1);
-        Words<W> nd = load_words_ro<W>(orow(plane + yprev));
-        Words<W> c = load_words_ro<W>(oth + (plane + y0) * p.pitch);
+        Words<W> nd = downs(load_words_ro<W>(orow(plane + yprev)));
+        Words<W> c = downs(load_words_ro<W>(oth + (plane + y0) * p.pitch));
         for (int y = y0; y < y1; ++y) {
             const long long row = plane + y;
             const long long ynext = NDIM == 2 ? y + 1 : (y + 1 == ly ? 0 : y + 1);
-            const Words<W> nu = load_words_ro<W>(orow(plane + ynext));
+            const Words<W> nu = downs(load_words_ro<W>(orow(plane + ynext)));
             Words<W> zu = nu, zd = nd;
             if constexpr (NDIM == 3) {  // planes z +- 1: plane -1 and plane lz are the halos
-                zu = load_words_ro<W>(orow(row + ly));
-                zd = load_words_ro<W>(orow(row - ly));
+                zu = downs(load_words_ro<W>(orow(row + ly)));
+                zd = downs(load_words_ro<W>(orow(row - ly)));
             }
             const int par = (g.par0 + y + z + (int)p.color) & 1;
             const u32 edge =
-                (u32)(uint8_t)__ldg(p.other + row * p.pitch + edge_index(p, par, j0, wv));
+                (u32)(uint8_t)__ldg(p.other + row * p.pitch + edge_index(p, par, j0, wv)) & kBit2;
             const Words<W> s = load_words<W>(p.own + row * p.pitch + j0);
-            const Words<W> ns = int8_update<V, NDIM, RULE, true, MEAS, false>(
-                p, g.row0 + row, par, j0, wv, s, c, nu, nd, zu, zd, edge, stab, m_acc, e_acc);
+            const Words<W> ns = int8_update<V, NDIM, RULE, true, MEAS>(
+                DrawSites<NDIM>{p, site_counter(p, g.row0 + row, j0)}, par, wv, s, c, nu, nd, zu, zd,
+                edge, rt, m_acc, e_acc);
             if constexpr (RULE != kObserve) store_words<W>(p.own + row * p.pitch + j0, ns);
             nd = c;
             c = nu;
@@ -311,9 +309,8 @@ static void launch_int8_slab_rule(int rule, const Int8Half& p, const SlabGeo& g,
     auto go = [&](auto kernel) { launch_pdl(kernel, dim3(grid), dim3(256), st, p, g); };
     switch (rule) {
     case kMetroFast: go(int8_slab_kernel<NDIM, kMetroFast, MEAS>); break;
-    case kHeatFast: go(int8_slab_kernel<NDIM, kHeatFast, MEAS>); break;
+    case kHeat: go(int8_slab_kernel<NDIM, kHeat, MEAS>); break;
     case kMetroGeneric: go(int8_slab_kernel<NDIM, kMetroGeneric, MEAS>); break;
-    case kHeatGeneric: go(int8_slab_kernel<NDIM, kHeatGeneric, MEAS>); break;
     default: go(int8_slab_kernel<NDIM, kObserve, true>); break;
     }
 }

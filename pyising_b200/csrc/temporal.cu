@@ -10,8 +10,7 @@
 // same random numbers, keyed by (site, sweep, colour) as everywhere else, so every result is
 // bit-identical to four single half-sweeps.
 //
-// Conditions (temporal_ok): int8 2D, a fast decision rule, rows a multiple of 16 bytes (no
-// padding, whole 16-byte chunks), Ly a multiple of kTbBand and at least kTbRows (no row twice
+// Conditions (temporal_ok): int8 2D, rows a multiple of 16 bytes (no padding, whole 16-byte chunks), Ly a multiple of kTbBand and at least kTbRows (no row twice
 // in a tile), the tile within the shared memory of a CTA.  Unmeasured sweeps only: measured
 // ones run the single half-sweep kernels.
 #include "capi_internal.h"
@@ -79,12 +78,9 @@ __global__ void __launch_bounds__(kTbThreads) int8_temporal_kernel(const Int8Hal
 {
     constexpr int V = kTbChunk;
     extern __shared__ __align__(16) int8_t tile[];  // [colour][kTbRows][lh]
-    __shared__ u32 stab[8];
+    __shared__ u32 rt[kLookupWords];  // the lookup table of the decisions
     Int8Half p = p_in;
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int i = 0; i < 7; ++i) stab[i] = p.table[i];
-    }
+    if (threadIdx.x == 0) fill_lookup<2, RULE>(rt, p.table);
     pdl_wait();  // the previous launch of the stream has completed
     pdl_trigger();
     resolve_ctl(p);  // p.t: the sweep of the first half-sweep (colour 0)
@@ -119,13 +115,14 @@ __global__ void __launch_bounds__(kTbThreads) int8_temporal_kernel(const Int8Hal
             gr = gr < 0 ? gr + ly : (gr >= ly ? gr - ly : gr);
             const int par = (gr + color) & 1;
             const Words<V / 4> s = lds_words<V>(own + tr * lh + j0);
-            const Words<V / 4> c = lds_words<V>(oth + tr * lh + j0);
-            const Words<V / 4> nu = lds_words<V>(oth + (tr + 1) * lh + j0);
-            const Words<V / 4> nd = lds_words<V>(oth + (tr - 1) * lh + j0);
+            const Words<V / 4> c = downs(lds_words<V>(oth + tr * lh + j0));
+            const Words<V / 4> nu = downs(lds_words<V>(oth + (tr + 1) * lh + j0));
+            const Words<V / 4> nd = downs(lds_words<V>(oth + (tr - 1) * lh + j0));
             const int je = par ? (j0 + V == lh ? 0 : j0 + V) : (j0 == 0 ? lh - 1 : j0 - 1);
-            const u32 edge = (u32)(uint8_t)oth[tr * lh + je];
-            const Words<V / 4> ns = int8_update<V, 2, RULE, false, false, false>(
-                q, gr, par, j0, V / 4, s, c, nu, nd, nu, nd, edge, stab, m_acc, e_acc);
+            const u32 edge = (u32)(uint8_t)oth[tr * lh + je] & kBit2;
+            const Words<V / 4> ns = int8_update<V, 2, RULE, false, false>(
+                DrawSites<2>{q, site_counter(q, gr, j0)}, par, V / 4, s, c, nu, nd, nu, nd, edge, rt,
+                m_acc, e_acc);
             sts_words<V>(own + tr * lh + j0, ns);
         }
         __syncthreads();
@@ -142,8 +139,7 @@ __global__ void __launch_bounds__(kTbThreads) int8_temporal_kernel(const Int8Hal
 bool temporal_ok(const ising_sim* h)
 {
     return h->variant == ISING_VARIANT_INT8 && h->ndim == 2 &&
-           (h->rule == kMetroFast || h->rule == kHeatFast) && h->lh % 16 == 0 &&
-           h->pitch == h->lh && h->ly % kTbBand == 0 && h->ly >= kTbRows &&
+           h->lh % 16 == 0 && h->pitch == h->lh && h->ly % kTbBand == 0 && h->ly >= kTbRows &&
            2 * kTbRows * h->lh <= kTbMaxSmem;
 }
 
@@ -198,8 +194,11 @@ static cudaError_t launch_int8_temporal(const ising_sim* h, u32 t, const unsigne
         cfg.numAttrs = 1;
         return cudaLaunchKernelEx(&cfg, kernel, p, i0, i1, o0, o1);
     };
-    return h->rule == kHeatFast ? launch(int8_temporal_kernel<kHeatFast>)
-                                : launch(int8_temporal_kernel<kMetroFast>);
+    switch (h->rule) {
+    case kMetroFast: return launch(int8_temporal_kernel<kMetroFast>);
+    case kHeat: return launch(int8_temporal_kernel<kHeat>);
+    default: return launch(int8_temporal_kernel<kMetroGeneric>);
+    }
 }
 
 int temporal_scratch(ising_sim* h)
