@@ -111,14 +111,15 @@ int ising_half_sweep(ising_sim* h, int color, uint64_t t);
 /* How ising_sweep issues its half-sweeps (no counterpart in the reference, which launches one
  * kernel per half-sweep from Python):
  *   ISING_SCHEDULE_AUTO       graphs for whole chunks of sweeps, launches for the rest (the
- *                             temporal tiles below for eligible lattices up to 1024^2);
+ *                             temporal tiles below for 2D lattices of up to 6.5M int8 or 16M
+ *                             packed sites per colour);
  *   ISING_SCHEDULE_LAUNCHES   one kernel launch per half-sweep;
  *   ISING_SCHEDULE_GRAPHS     replayed CUDA graphs of whole chunks of sweeps;
  *   ISING_SCHEDULE_PERSISTENT one cooperative launch for all sweeps (2D int8; others fall back):
  *                             bands of rows wait only for their neighbours, every wait bounded;
- *   ISING_SCHEDULE_TEMPORAL   graphs whose launches each run two unmeasured sweeps on
- *                             shared-memory tiles with recomputed halos (small 2D int8
- *                             lattices with rows a multiple of 16 bytes; others fall back).
+ *   ISING_SCHEDULE_TEMPORAL   graphs whose launches each run several half-sweeps on
+ *                             shared-memory tiles with recomputed halos (2D lattices whose
+ *                             rows fit; others fall back).
  * All schedules give identical results.  test_mute_band >= 0 makes that band of a persistent
  * run stop publishing its progress, so its neighbours' bounded waits expire: the sweep then
  * reports ISING_ERR_TIMEOUT (the lattice is no longer valid); pass -1 otherwise. */

@@ -169,16 +169,23 @@ void clear_graphs(ising_sim* h)
     h->graphs.clear();
 }
 
-// Two unmeasured sweeps per launch on shared-memory tiles: when asked for, and by default for
-// eligible lattices of up to 512K sites per colour (1024^2), where a half-sweep is too short to
-// hide its launch (larger ones measured faster with single half-sweeps).
-constexpr long long kTemporalAutoSites = 512 * 1024;
+// Several half-sweeps per launch on shared-memory tiles: when asked for, and by default for
+// eligible lattices up to these many sites per colour (flips/ns, tiles / single half-sweeps).  A
+// launch knob of the single half-sweeps set by hand selects those (for int8 above kTemporalKnobs
+// sites).
+constexpr long long kTemporalInt8 = 6400 * 1024;  // 3500x3584 853 / 837, 4096^2 900 / 940
+constexpr long long kTemporalMsc = 4000 * 4096;   // 6000x5248 2202 / 1942, 6144^2 2309 / 2326
+constexpr long long kTemporalKnobs = 512 * 1024;
 
 static bool use_temporal(const ising_sim* h)
 {
     if (!temporal_ok(h)) return false;
     if (h->schedule == ISING_SCHEDULE_TEMPORAL) return true;
-    return h->schedule == ISING_SCHEDULE_AUTO && h->rows * (long long)h->lh <= kTemporalAutoSites;
+    if (h->schedule != ISING_SCHEDULE_AUTO) return false;
+    const long long sites = h->rows * (long long)h->lh;
+    if (h->variant == ISING_VARIANT_MSC)
+        return h->msc_kernel == 0 && h->msc_waves == 1 && sites <= kTemporalMsc;
+    return sites <= (h->band == 0 && h->vw == 16 ? kTemporalInt8 : kTemporalKnobs);
 }
 
 // The captured chunk of G sweeps of this handle: 2G half-sweeps with counters relative to the
@@ -194,14 +201,12 @@ static int chunk_graph(ising_sim* h, int64_t G, bool measured, cudaGraphExec_t* 
     cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamBeginCapture");
     int rc = ISING_OK;
-    const bool tb = use_temporal(h);
-    const int K = temporal_sweeps();
     int64_t s = 0;
-    if (tb) {  // K unmeasured sweeps per launch, up to the measured last sweep
-        const int64_t runs = (G - (measured ? 1 : 0)) / K;
-        const cudaError_t le = launch_temporal_run(h, 0u, runs, ctl);
+    if (use_temporal(h)) {
+        const cudaError_t le = launch_temporal_run(
+            h, 0u, G, measured ? (unsigned long long*)h->d_series : nullptr, ctl);
         if (le != cudaSuccess) rc = cuda_fail(le, "temporal half-sweeps");
-        s = runs * K;
+        s = G;
     }
     for (; s < G && rc == ISING_OK;) {
         unsigned long long* m =
@@ -759,25 +764,22 @@ int ising_sweep(ising_sim* h, uint64_t t0, int64_t n_sweeps, int64_t measure_eve
             s0 = n_sweeps;
         }
     }
-    const bool tb = use_temporal(h);
-    const int K = temporal_sweeps();
-    // sweeps s .. s + K - 1 hold no measurement
-    auto unmeasured = [&](int64_t s) {
-        if (measure_every <= 0) return true;
-        for (int i = 0; i < K; ++i)
-            if ((s + i + 1) % measure_every == 0) return false;
-        return true;
-    };
+    while (use_temporal(h) && s0 < n_sweeps) {  // up to the next measured sweep, or the end
+        int64_t run = n_sweeps - s0;
+        bool meas = false;
+        if (measure_every > 0 && measure_every - s0 % measure_every <= run) {
+            run = measure_every - s0 % measure_every;
+            meas = true;
+        }
+        TRY_CUDA(launch_temporal_run(h, (u32)(t0 + (uint64_t)s0), run,
+                                     meas ? (unsigned long long*)(h->d_series + 2 * k) : nullptr,
+                                     nullptr));
+        s0 += run;
+        if (meas) ++k;
+    }
     for (int64_t s = s0; s < n_sweeps; ++s) {
         const u32 t = (u32)(t0 + (uint64_t)s);
         const bool meas = measure_every > 0 && (s + 1) % measure_every == 0;
-        if (tb && s + K <= n_sweeps && unmeasured(s)) {
-            int64_t runs = 0;  // consecutive launches of K unmeasured sweeps from s
-            while (s + (runs + 1) * K <= n_sweeps && unmeasured(s + runs * K)) ++runs;
-            TRY_CUDA(launch_temporal_run(h, t, runs, nullptr));
-            s += runs * K - 1;
-            continue;
-        }
         unsigned long long* m = meas ? (unsigned long long*)(h->d_series + 2 * k) : nullptr;
         int rc = half_sweep(h, 0, t, nullptr, nullptr);
         if (rc == ISING_OK) rc = half_sweep(h, 1, t, m, nullptr);

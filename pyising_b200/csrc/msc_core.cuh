@@ -230,6 +230,38 @@ __device__ __forceinline__ void intake_load(const MscHalf& p, long long w, bool 
     }
 }
 
+// What one Philox block decides of 32 lanes, apart from the blocks before it: eq = undecided after
+// both its levels, lt = accepted by them.  Blocks compose: (eq1, lt1) then (eq2, lt2) is
+// (eq1 & eq2, lt1 | (eq1 & lt2)).
+struct HalfBlock {
+    u32 eq, lt;
+};
+
+__device__ __forceinline__ HalfBlock half_block(u32 re, u32 ro, const uint4& m, u32 a1)
+{
+    const u32 tme = (a1 & m.x) | (~a1 & m.y);
+    const u32 tmo = (a1 & m.z) | (~a1 & m.w);
+    const u32 eq = ~(re ^ tme);
+    HalfBlock h;
+    h.lt = (~re & tme) | (eq & ~ro & tmo);
+    h.eq = eq & ~(ro ^ tmo);
+    return h;
+}
+
+// What G consecutive lanes decide of their word, lane g having the block(s) after lane g - 1's:
+// the result is in all of them.
+template <int G>
+__device__ __forceinline__ void compose_lanes(HalfBlock& h)
+{
+#pragma unroll
+    for (int s = 1; s < G; s <<= 1) {
+        const u32 eq = __shfl_xor_sync(0xFFFFFFFFu, h.eq, s);
+        const u32 lt = __shfl_xor_sync(0xFFFFFFFFu, h.lt, s);
+        h.lt = (threadIdx.x & (u32)s) ? lt | (eq & h.lt) : h.lt | (h.eq & lt);
+        h.eq &= eq;
+    }
+}
+
 // The end of a warp's work: the at most 32 stack entries left take one lane each, and each lane
 // draws its entry's Philox blocks one after another until the entry is decided, without going
 // back to the stack.  Draining by stack passes instead (pop, one block, push back the undecided)
