@@ -8,11 +8,12 @@
 // own series slot.  The random numbers depend only on (site, sweep, colour, seed), so each
 // lattice is bit-identical to running it alone with the single-lattice kernels.
 //
-// Work items are tiles of ~16K int8 sites (whole rows) or ~4K packed words; items of one
-// kernel class (variant, chunk width, dims, decision rule) share a launch; a block walks its
-// items grid-stride.  The host engine decides membership deterministically from sweep counts,
-// so it never waits for the device except to hand results back (events) and to bound how far
-// it runs ahead.
+// Lattices of one kernel class (variant, dims, decision rule, padded or not) share a launch, and
+// classes run side by side on streams of their own (measured on one B200, 21 served jobs of five
+// classes: 21.4 ms one after another, 15.9 side by side, 11.7 with small classes on one chunk or
+// word per thread).  The host engine decides membership deterministically from sweep counts, so
+// it never waits for the device except to hand results back (events) and to bound how far it runs
+// ahead.
 #include <algorithm>
 #include <climits>
 #include <chrono>
@@ -50,6 +51,16 @@ struct BatchLattice {
 constexpr long long kInt8ItemMin = 512, kInt8ItemMax = 4096;    // band slots
 constexpr long long kMscItemMin = 2048, kMscItemMax = 16384;    // words
 constexpr long long kItemsPerSlot = 6;  // default of the ISING_KNOB_ITEMS_PER_SLOT knob
+// Chunk-rows (2D, 3D) and msc words per SM below which a class runs one chunk or word per thread.
+// Measured on one B200 against bands and word ranges (flips/ns of a batch): 64 x 256^2 398 / 353,
+// 8 x 1000x1048 640 / 524, 12 x 64^3 heat bath 409 / 303, 3D heat bath 56^3..248^3 (707,000
+// chunks) 656 / 607, msc 128^2..2688^2 1541 / 690, 6 x msc 4096^2 (786,000 words) 2328 / 2278.
+// (16 x 1024^2, 524,288 chunks: 709 / 670; 32 lattices of 755,000 chunks: 633 / 653.)
+constexpr long long kOneUnits2 = 4000, kOneUnits3 = 6000, kOneWords = 6000;
+// Blocks of 256 band slots per resident block that the band height of a class leaves: two keep the
+// bands two rows high (which fixes the row parity in the code) where six, as for the work items,
+// gave bands of one row: 32 lattices of 755,000 chunks 602 -> 653, 2 x 4096^2 851 -> 974.
+constexpr long long kBandBlocks = 2;
 constexpr int kBandCap = 8;             // default of the ISING_KNOB_BAND knob (batch)
 
 // Item size for `total` units of work over `slots` resident blocks, `per_slot` items each.
@@ -95,6 +106,47 @@ struct Int8LaunchN {
 using Int8Launch = Int8LaunchN<kInt8PerLaunch>;
 static_assert(sizeof(Int8Launch) <= 32764, "kernel parameter block over the 32 KB limit");
 
+// The lattice of this block: the last one whose block_begin is not beyond it.
+template <class Desc>
+__device__ __forceinline__ int find_lattice(const Desc* lat, int n)
+{
+    const int b = (int)blockIdx.x;
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (lat[mid].block_begin <= b) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// The half-sweep of lattice L at `epoch`; meas: it ends a measured sweep.
+__device__ __forceinline__ Int8Half lattice_half(const Int8Desc& L, long long epoch, int v, bool& meas)
+{
+    const u32 color = (u32)(epoch & 1);
+    const u32 s = (u32)((epoch - L.join_epoch) >> 1);  // sweeps done (< 2^31)
+    meas = color == 1 && L.every > 0 && ((s + 1u) % (u32)L.every) == 0;
+    Int8Half p;
+    p.own = static_cast<int8_t*>(L.c[color]);
+    p.other = static_cast<const int8_t*>(L.c[color ^ 1]);
+    p.rows = L.rows;
+    p.lh = L.lh;
+    p.ly = L.ly;
+    p.lz = L.lz;
+    p.cpr = L.cpr;
+    p.pitch = L.pitch;
+    p.vw = v;
+    p.t = L.t0 + s;
+    p.color = color;
+    p.k0 = L.k0;
+    p.k1 = L.k1;
+    p.meas = meas ? reinterpret_cast<unsigned long long*>(
+                        L.series + 2 * ((s + 1u) / (u32)L.every - 1u))
+                  : nullptr;
+    p.ctl = nullptr;
+    return p;
+}
+
 template <int V, int NDIM, int RULE, bool MIXED, bool MEAS>
 __device__ __forceinline__ void batch_int8_slots(const Int8Half& p, const Int8Desc& L, u32 s0,
                                                  u32 s1, const u32* rt, long long& m_acc,
@@ -128,40 +180,13 @@ __global__ void __launch_bounds__(256, ISING_BATCH_MIN_BLOCKS)
     // class's previous half-sweep has completed too), then let the next launch start
     pdl_wait();
     pdl_trigger();
-    const int b = (int)blockIdx.x;
-    int lo = 0, hi = P.n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (P.lat[mid].block_begin <= b) lo = mid;
-        else hi = mid - 1;
-    }
-    const Int8Desc& L = P.lat[lo];
+    const Int8Desc& L = P.lat[find_lattice(P.lat, P.n)];
     if (threadIdx.x == 0) fill_lookup<NDIM, RULE>(rt, L.table);
     __syncthreads();
     const long long epoch = P.epoch + (P.epoch_base ? *P.epoch_base : 0);
-    const u32 color = (u32)(epoch & 1);
-    const u32 s = (u32)((epoch - L.join_epoch) >> 1);  // sweeps done (< 2^31)
-    const bool meas = color == 1 && L.every > 0 && ((s + 1u) % (u32)L.every) == 0;
-    Int8Half p;
-    p.own = static_cast<int8_t*>(L.c[color]);
-    p.other = static_cast<const int8_t*>(L.c[color ^ 1]);
-    p.rows = L.rows;
-    p.lh = L.lh;
-    p.ly = L.ly;
-    p.lz = L.lz;
-    p.cpr = L.cpr;
-    p.pitch = L.pitch;
-    p.vw = V;
-    p.t = L.t0 + s;
-    p.color = color;
-    p.k0 = L.k0;
-    p.k1 = L.k1;
-#pragma unroll
-    for (int i = 0; i < 7; ++i) p.table[i] = L.table[i];
-    p.meas = meas ? reinterpret_cast<unsigned long long*>(
-                        L.series + 2 * ((s + 1u) / (u32)L.every - 1u))
-                  : nullptr;
-    p.ctl = nullptr;
+    bool meas;
+    const Int8Half p = lattice_half(L, epoch, V, meas);
+    const int b = (int)blockIdx.x;
     const u32 s0 = (u32)(b - L.block_begin) * (u32)L.per_block;
     const u32 s1 = s0 + (u32)L.per_block < (u32)L.nslots ? s0 + (u32)L.per_block : (u32)L.nslots;
     long long m_acc = 0, e_acc = 0;
@@ -173,7 +198,143 @@ __global__ void __launch_bounds__(256, ISING_BATCH_MIN_BLOCKS)
     }
 }
 
+// One chunk per thread, for classes with too few chunks to give every thread a band: as
+// int8_one_kernel, the random numbers are drawn before the class's previous half-sweep is done.
+constexpr int kOneThreads = 128;
+
+template <int NDIM, int RULE, bool MIXED, int N>
+__global__ void __launch_bounds__(kOneThreads)
+    batch_int8_one_kernel(const __grid_constant__ Int8LaunchN<N> P)
+{
+    constexpr int V = 16, W = 4;
+    __shared__ u32 rt[kLookupWords];  // the lookup table of the decisions
+    const Int8Desc& L = P.lat[find_lattice(P.lat, P.n)];
+    if (threadIdx.x == 0) fill_lookup<NDIM, RULE>(rt, L.table);
+    // (the device epoch counter changes between graph replays only)
+    const long long epoch = P.epoch + (P.epoch_base ? *P.epoch_base : 0);
+    bool meas;
+    const Int8Half p = lattice_half(L, epoch, V, meas);
+    const u32 slot = (u32)((int)blockIdx.x - L.block_begin) * kOneThreads + threadIdx.x;
+    const u32 row = fast_div(slot, (u32)L.cpr, L.cpr_magic);
+    const int j0 = (int)(slot - row * (u32)L.cpr) * V;
+    int z = 0, y = (int)row;
+    if constexpr (NDIM == 3) {
+        z = (int)fast_div(row, (u32)L.bpp, L.bpp_magic);
+        y = (int)(row - (u32)z * (u32)L.bpp);
+    }
+    const DrawSites<NDIM> sites{p, site_counter(p, row, j0)};
+    u32x4 r[W];
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+        r[k] = sites(k);
+        asm volatile("" : "+r"(r[k].x), "+r"(r[k].y), "+r"(r[k].z), "+r"(r[k].w));
+    }
+    __syncthreads();
+    pdl_wait();
+    pdl_trigger();
+    auto drawn = [&](int k) { return r[k]; };
+    long long m_acc = 0, e_acc = 0;
+    const bool valid = slot < (u32)L.nslots;
+    if (meas) {
+        if (valid)
+            int8_chunk<V, NDIM, RULE, false, MIXED, true>(p, drawn, row, y, z, j0, rt, m_acc, e_acc);
+        block_accumulate2(m_acc, e_acc, p.meas);
+    } else if (valid) {
+        int8_chunk<V, NDIM, RULE, false, MIXED, false>(p, drawn, row, y, z, j0, rt, m_acc, e_acc);
+    }
+}
+
 // ------------------------------------------------------------------------------ msc -------
+// Small msc classes run one word per thread, the lattice descriptors in the launch's parameters
+// as for int8 and kOneCalls Philox blocks per word drawn before the class's previous half-sweep is
+// done; larger ones walk word ranges with a work stack (batch_msc_kernel).
+struct MscDesc {
+    u64* c[2];
+    long long* series;     // (M, E) pairs, or nullptr
+    long long join_epoch;  // even epoch of the first half-sweep
+    u64 nw_magic;          // ceil(2^64 / nw)
+    int every;             // measurement interval in sweeps (0 = none)
+    int rows, nw, nw_shift;
+    u32 t0, k0, k1, thr4, thr8;
+    int block_begin;       // first block of this lattice in the launch
+};
+
+template <int N>
+struct MscLaunchN {
+    long long epoch;
+    const long long* epoch_base;
+    int n;
+    int pad;
+    MscDesc lat[N];
+};
+using MscLaunch = MscLaunchN<kInt8PerLaunch>;
+static_assert(sizeof(MscLaunch) <= 32764, "kernel parameter block over the 32 KB limit");
+
+constexpr int kOneCalls = 6;
+
+template <int N>
+__global__ void __launch_bounds__(kOneThreads)
+    batch_msc_one_kernel(const __grid_constant__ MscLaunchN<N> P)
+{
+    __shared__ uint4 lvmask[16];
+    const MscDesc& L = P.lat[find_lattice(P.lat, P.n)];
+    if (threadIdx.x < 16) lvmask[threadIdx.x] = level_masks(L.thr4, L.thr8, threadIdx.x);
+    const long long epoch = P.epoch + (P.epoch_base ? *P.epoch_base : 0);
+    const u32 color = (u32)(epoch & 1);
+    const u32 s = (u32)((epoch - L.join_epoch) >> 1);  // sweeps done (< 2^31)
+    const bool meas = color == 1 && L.every > 0 && ((s + 1u) % (u32)L.every) == 0;
+    MscHalf p;
+    p.own = L.c[color];
+    p.other = L.c[color ^ 1];
+    p.rows = L.rows;
+    p.nw = L.nw;
+    p.t = L.t0 + s;
+    p.color = color;
+    p.k0 = L.k0;
+    p.k1 = L.k1;
+    p.nw_magic = L.nw_magic;
+    const u32 w = (u32)((int)blockIdx.x - L.block_begin) * kOneThreads + threadIdx.x;
+    u32x4 r[kOneCalls];
+#pragma unroll
+    for (int b = 0; b < kOneCalls; ++b) {
+        r[b] = philox4x32_10<true>(w, p.t, color, 1u + (u32)b, p.k0, p.k1);
+        asm volatile("" : "+r"(r[b].x), "+r"(r[b].y), "+r"(r[b].z), "+r"(r[b].w));
+    }
+    __syncthreads();
+    pdl_wait();
+    pdl_trigger();
+    long long m_acc = 0, e_acc = 0;
+    const bool valid = w < (u32)L.rows * (u32)L.nw;
+    if (valid) {
+        IntakeLoads I;
+        intake_load(p, w, true, L.nw, L.nw_shift, I);
+        const bool par = ((I.y + (int)color) & 1) != 0;
+        const u64 hz = par ? ((I.c >> 1) | (I.side << 63)) : ((I.c << 1) | (I.side >> 63));
+        const HalfSlices al = slice_half((u32)I.o, (u32)I.c, (u32)hz, (u32)I.up, (u32)I.dn);
+        const HalfSlices ah = slice_half((u32)(I.o >> 32), (u32)(I.c >> 32), (u32)(hz >> 32),
+                                         (u32)(I.up >> 32), (u32)(I.dn >> 32));
+        u32 ul = ~al.a2, uh = ~ah.a2, accl = 0, acch = 0;
+#pragma unroll
+        for (int b = 0; b < kOneCalls; ++b)
+            block_levels(r[b], lvmask[b], al.a1, ah.a1, ul, uh, accl, acch);
+        for (u32 lp = kOneCalls; lp < 16u && (ul | uh) != 0; ++lp) {
+            const u32x4 more = philox4x32_10<true>(w, p.t, color, 1u + lp, p.k0, p.k1);
+            block_levels(more, lvmask[lp], al.a1, ah.a1, ul, uh, accl, acch);
+        }
+        const u64 ns = I.o ^ ((u64)(al.a2 | accl) | ((u64)(ah.a2 | acch) << 32));
+        p.own[w] = ns;
+        if (meas) {
+            const int anti = __popcll(ns ^ I.c) + __popcll(ns ^ hz) + __popcll(ns ^ I.up) +
+                             __popcll(ns ^ I.dn);
+            m_acc = 2 * (__popcll(ns) + __popcll(I.c)) - 128;
+            e_acc = 2 * anti - 256;
+        }
+    }
+    if (meas)
+        block_accumulate2(m_acc, e_acc, reinterpret_cast<unsigned long long*>(
+                                            L.series + 2 * ((s + 1u) / (u32)L.every - 1u)));
+}
+
 struct BatchItem {
     int lat;
     int pad;
@@ -271,6 +432,13 @@ struct KernelClass {
     }
 };
 
+// The launches of one int8 class.
+struct Int8Class {
+    KernelClass kc;
+    bool one;  // one chunk per thread
+    std::vector<Int8Launch> launches;
+};
+
 class Engine {
 public:
     Engine(int device, int64_t budget) : device_(device), budget_(budget) {}
@@ -303,6 +471,7 @@ public:
     ~Engine()
     {
         cudaSetDevice(device_);
+        for (Aux& a : aux_) cudaStreamSynchronize(a.stream);
         if (stream_) cudaStreamSynchronize(stream_);
         for (auto& kv : jobs_) free_job(*kv.second);
         if (d_lats_) cudaFreeAsync(d_lats_, stream_);
@@ -316,6 +485,11 @@ public:
         if (d_epoch_) cudaFree(d_epoch_);
         for (auto& kv : pinned_free_) cudaFreeHost(kv.second);
         for (cudaEvent_t ev : epoch_events_) cudaEventDestroy(ev);
+        for (Aux& a : aux_) {
+            cudaEventDestroy(a.event);
+            cudaStreamDestroy(a.stream);
+        }
+        if (fork_event_) cudaEventDestroy(fork_event_);
         if (stream_) cudaStreamDestroy(stream_);
         if (pool_) cudaMemPoolDestroy(pool_);
         cudaGetLastError();
@@ -391,7 +565,8 @@ public:
         if (e != cudaSuccess) return cuda_fail(e, "batch launch");
         ++epoch_;
         if ((epoch_ & 1) == 0) {
-            int rc = retire();
+            int rc = join();
+            if (rc == ISING_OK) rc = retire();
             if (rc != ISING_OK) return rc;
             rc = throttle();
             if (rc != ISING_OK) return rc;
@@ -424,6 +599,8 @@ public:
 
     int wait_finishing()
     {
+        const int rc = join();
+        if (rc != ISING_OK) return rc;
         cudaError_t e = cudaStreamSynchronize(stream_);
         if (e != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
         poll();
@@ -622,6 +799,8 @@ private:
     // work items in device memory.
     int rebuild()
     {
+        int jrc = join();
+        if (jrc != ISING_OK) return jrc;
         std::vector<BatchLattice> lats;              // msc lattices
         std::map<KernelClass, std::vector<Int8Desc>> int8_descs;
         std::map<KernelClass, long long> class_units;  // chunk-rows (int8) or words (msc)
@@ -677,19 +856,25 @@ private:
             }
         }
         // int8: the class's band height is the longest power of two up to the band cap that
-        // still leaves items_per_slot blocks of one slot per thread per resident block; blocks
-        // of a lattice hold per_block slots, sized the same way
+        // still leaves kBandBlocks (or items_per_slot, if fewer) blocks of one slot per thread per
+        // resident block; blocks of a lattice hold per_block slots, items_per_slot blocks per
+        // resident block
         int8_launches_.clear();
         for (auto& kv : int8_descs) {
             const KernelClass& kc = kv.first;
             const long long units = class_units[kc];
-            const long long want = items_per_slot_ * 256 * slots(kc);
             int band = 1;
             while (band * 2 <= band_cap_) band *= 2;
+            const long long want = std::min(items_per_slot_, kBandBlocks) * 256 * slots(kc);
             while (band > 1 && units / band < want) band >>= 1;
             long long per = item_size(units / band, slots(kc), items_per_slot_, kInt8ItemMin,
                                       kInt8ItemMax);
             per = (per + 255) / 256 * 256;
+            const bool one = units < (kc.ndim == 3 ? kOneUnits3 : kOneUnits2) * sms_;
+            if (one) {
+                band = 1;
+                per = kOneThreads;
+            }
             std::vector<Int8Launch> launches;
             for (size_t i = 0; i < kv.second.size(); ++i) {
                 if (i % kInt8PerLaunch == 0) {
@@ -712,10 +897,41 @@ private:
                 D.block_begin = prev;
                 P.lat[P.n++] = D;
             }
-            int8_launches_.emplace_back(kc, std::move(launches));
+            int8_launches_.push_back(Int8Class{kc, one, std::move(launches)});
         }
-        // msc: work items of whole 256-word runs over the class's lattices
+        // msc: one word per thread for small totals, else work items of whole 256-word runs over
+        // the class's lattices
+        msc_one_.clear();
         std::map<KernelClass, std::vector<BatchItem>> by_class;
+        if (!msc_of.empty() && class_units[msc_of[0].first] < kOneWords * sms_) {
+            for (const auto& m : msc_of) {
+                if (msc_one_.empty() || msc_one_.back().n == kInt8PerLaunch) {
+                    msc_one_.emplace_back();
+                    memset(&msc_one_.back(), 0, sizeof(MscLaunch));
+                }
+                MscLaunch& P = msc_one_.back();
+                const BatchLattice& L = lats[m.second];
+                MscDesc D;
+                memset(&D, 0, sizeof D);
+                D.c[0] = static_cast<u64*>(L.c[0]);
+                D.c[1] = static_cast<u64*>(L.c[1]);
+                D.series = L.series;
+                D.join_epoch = L.join_epoch;
+                D.nw_magic = L.nw_magic;
+                D.every = L.every;
+                D.rows = L.rows;
+                D.nw = L.nw;
+                D.nw_shift = L.nw_shift;
+                D.t0 = L.t0;
+                D.k0 = L.k0;
+                D.k1 = L.k1;
+                D.thr4 = L.table[3];
+                D.thr8 = L.table[4];
+                D.block_begin = P.n ? (int)msc_grid(P) : 0;
+                P.lat[P.n++] = D;
+            }
+            msc_of.clear();
+        }
         for (const auto& m : msc_of) {
             const KernelClass& kc = m.first;
             const BatchLattice& L = lats[m.second];
@@ -736,7 +952,58 @@ private:
         if (rc == ISING_OK)
             rc = upload(items.data(), items.size() * sizeof(BatchItem), (void**)&d_items_, &items_cap_);
         dirty_ = false;
+        if (rc == ISING_OK) rc = plan_streams();
         return rc;
+    }
+
+    // Every class advances on a stream of its own when there are several: their lattices are
+    // independent, and a class alone often leaves most of the GPU waiting.  The engine's stream
+    // waits for all of them at every sweep (join), they wait for it only after it did something
+    // (fork): admissions, results, work lists, graph chunks.
+    int plan_streams()
+    {
+        size_t n = int8_launches_.size() + (msc_one_.empty() ? 0 : 1) + classes_.size();
+        n_aux_ = n > 1 ? n : 0;
+        while (aux_.size() < n_aux_) {
+            Aux a;
+            cudaError_t e = cudaStreamCreateWithFlags(&a.stream, cudaStreamNonBlocking);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&a.event, cudaEventDisableTiming);
+            if (e != cudaSuccess) {
+                if (a.stream) cudaStreamDestroy(a.stream);
+                return cuda_fail(e, "batch class stream");
+            }
+            aux_.push_back(a);
+        }
+        if (n_aux_ && !fork_event_) {
+            const cudaError_t e = cudaEventCreateWithFlags(&fork_event_, cudaEventDisableTiming);
+            if (e != cudaSuccess) return cuda_fail(e, "batch fork event");
+        }
+        forked_ = false;
+        return ISING_OK;
+    }
+
+    // The class streams wait for the engine's.
+    cudaError_t fork()
+    {
+        if (!n_aux_ || forked_) return cudaSuccess;
+        cudaError_t e = cudaEventRecord(fork_event_, stream_);
+        for (size_t i = 0; i < n_aux_ && e == cudaSuccess; ++i)
+            e = cudaStreamWaitEvent(aux_[i].stream, fork_event_, 0);
+        forked_ = e == cudaSuccess;
+        return e;
+    }
+
+    // The engine's stream waits for the class streams.
+    int join()
+    {
+        if (!joinable_) return ISING_OK;
+        for (size_t i = 0; i < n_aux_; ++i) {
+            cudaError_t e = cudaEventRecord(aux_[i].event, aux_[i].stream);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(stream_, aux_[i].event, 0);
+            if (e != cudaSuccess) return cuda_fail(e, "batch class join");
+        }
+        joinable_ = false;
+        return ISING_OK;
     }
 
     // Blocks of an int8 launch: the last lattice's block_begin plus its blocks.
@@ -744,6 +1011,13 @@ private:
     {
         const Int8Desc& L = P.lat[P.n - 1];
         return (unsigned)(L.block_begin + (L.nslots + L.per_block - 1) / L.per_block);
+    }
+
+    static unsigned msc_grid(const MscLaunch& P)
+    {
+        const MscDesc& L = P.lat[P.n - 1];
+        const long long words = (long long)L.rows * L.nw;
+        return (unsigned)(L.block_begin + (words + kOneThreads - 1) / kOneThreads);
     }
 
     // Resident blocks of a class's kernel on the whole device.
@@ -791,8 +1065,17 @@ private:
         return n_items < g ? n_items : g;
     }
 
-    template <int V, int NDIM, bool MIXED, int N>
-    cudaError_t launch_int8_cap(int rule, const Int8Launch& full)
+    template <int NDIM, int RULE, bool MIXED, int N>
+    cudaError_t launch_int8_kernel(bool one, const Int8LaunchN<N>& P, unsigned grid, cudaStream_t st)
+    {
+        if (one)
+            return launch_pdl(batch_int8_one_kernel<NDIM, RULE, MIXED, N>, dim3(grid),
+                              dim3(kOneThreads), st, P);
+        return launch_pdl(batch_int8_kernel<16, NDIM, RULE, MIXED, N>, dim3(grid), dim3(256), st, P);
+    }
+
+    template <int NDIM, bool MIXED, int N>
+    cudaError_t launch_int8_cap(const Int8Class& c, const Int8Launch& full, cudaStream_t st)
     {
         Int8LaunchN<N> P;
         P.epoch = full.epoch;
@@ -800,62 +1083,89 @@ private:
         P.n = full.n;
         P.pad = 0;
         memcpy(P.lat, full.lat, (size_t)full.n * sizeof(Int8Desc));
-        const dim3 grid(int8_grid(full)), block(256);
-        switch (rule) {
-        case kMetroFast:
-            return launch_pdl(batch_int8_kernel<V, NDIM, kMetroFast, MIXED, N>, grid, block, stream_, P);
-        case kHeat:
-            return launch_pdl(batch_int8_kernel<V, NDIM, kHeat, MIXED, N>, grid, block, stream_, P);
+        const unsigned grid = int8_grid(full);
+        switch (c.kc.rule) {
+        case kMetroFast: return launch_int8_kernel<NDIM, kMetroFast, MIXED, N>(c.one, P, grid, st);
+        case kHeat: return launch_int8_kernel<NDIM, kHeat, MIXED, N>(c.one, P, grid, st);
         case kMetroGeneric:
-            return launch_pdl(batch_int8_kernel<V, NDIM, kMetroGeneric, MIXED, N>, grid, block,
-                              stream_, P);
+            return launch_int8_kernel<NDIM, kMetroGeneric, MIXED, N>(c.one, P, grid, st);
         default: return cudaErrorInvalidValue;
         }
     }
 
-    template <int V, int NDIM, bool MIXED>
-    cudaError_t launch_int8_rule(int rule, const Int8Launch& P)
+    template <int NDIM, bool MIXED>
+    cudaError_t launch_int8_n(const Int8Class& c, const Int8Launch& P, cudaStream_t st)
     {
-        if (P.n <= 16) return launch_int8_cap<V, NDIM, MIXED, 16>(rule, P);
-        if (P.n <= 64) return launch_int8_cap<V, NDIM, MIXED, 64>(rule, P);
-        return launch_int8_cap<V, NDIM, MIXED, kInt8PerLaunch>(rule, P);
+        if (P.n <= 16) return launch_int8_cap<NDIM, MIXED, 16>(c, P, st);
+        if (P.n <= 64) return launch_int8_cap<NDIM, MIXED, 64>(c, P, st);
+        return launch_int8_cap<NDIM, MIXED, kInt8PerLaunch>(c, P, st);
     }
 
     // int8 rows are padded to 16 bytes, so the chunk width is always 16; lattices whose rows are
     // a multiple of 16 get the kernel without the partial-chunk code.
-    cudaError_t launch_int8(const KernelClass& kc, const Int8Launch& P)
+    cudaError_t launch_int8(const Int8Class& c, const Int8Launch& P, cudaStream_t st)
     {
-        if (kc.ndim == 3)
-            return kc.mixed ? launch_int8_rule<16, 3, true>(kc.rule, P)
-                            : launch_int8_rule<16, 3, false>(kc.rule, P);
-        return kc.mixed ? launch_int8_rule<16, 2, true>(kc.rule, P)
-                        : launch_int8_rule<16, 2, false>(kc.rule, P);
+        if (c.kc.ndim == 3)
+            return c.kc.mixed ? launch_int8_n<3, true>(c, P, st) : launch_int8_n<3, false>(c, P, st);
+        return c.kc.mixed ? launch_int8_n<2, true>(c, P, st) : launch_int8_n<2, false>(c, P, st);
     }
 
-    cudaError_t launch_msc(int off, int n, long long epoch, const long long* epoch_base)
+    template <int N>
+    cudaError_t launch_msc_one_cap(const MscLaunch& full, cudaStream_t st)
+    {
+        MscLaunchN<N> P;
+        P.epoch = full.epoch;
+        P.epoch_base = full.epoch_base;
+        P.n = full.n;
+        P.pad = 0;
+        memcpy(P.lat, full.lat, (size_t)full.n * sizeof(MscDesc));
+        return launch_pdl(batch_msc_one_kernel<N>, dim3(msc_grid(full)), dim3(kOneThreads), st, P);
+    }
+
+    cudaError_t launch_msc_one(const MscLaunch& P, cudaStream_t st)
+    {
+        if (P.n <= 16) return launch_msc_one_cap<16>(P, st);
+        if (P.n <= 64) return launch_msc_one_cap<64>(P, st);
+        return launch_msc_one_cap<kInt8PerLaunch>(P, st);
+    }
+
+    cudaError_t launch_msc(int off, int n, long long epoch, const long long* epoch_base,
+                           cudaStream_t st)
     {
         auto fn = batch_msc_kernel;
         const dim3 grid(grid_for((const void*)fn, n, kBatchWarps * 32)), block(kBatchWarps * 32);
-        fn<<<grid, block, 0, stream_>>>(d_lats_, d_items_ + off, n, epoch, epoch_base);
+        fn<<<grid, block, 0, st>>>(d_lats_, d_items_ + off, n, epoch, epoch_base);
         return cudaGetLastError();
     }
 
     // Every class's launches of one epoch (absolute, or relative to *epoch_base).
     cudaError_t launch_epoch(long long epoch, const long long* epoch_base)
     {
-        cudaError_t e = cudaSuccess;
+        cudaError_t e = fork();
+        size_t i = 0;
+        auto next_stream = [&] { return n_aux_ ? aux_[i++].stream : stream_; };
         for (auto& cl : int8_launches_) {
-            for (Int8Launch& P : cl.second) {
+            const cudaStream_t st = next_stream();
+            for (Int8Launch& P : cl.launches) {
                 P.epoch = epoch;
                 P.epoch_base = epoch_base;
-                e = launch_int8(cl.first, P);
-                if (e != cudaSuccess) return e;
+                if (e == cudaSuccess) e = launch_int8(cl, P, st);
+            }
+        }
+        if (!msc_one_.empty()) {
+            const cudaStream_t st = next_stream();
+            for (MscLaunch& P : msc_one_) {
+                P.epoch = epoch;
+                P.epoch_base = epoch_base;
+                if (e == cudaSuccess) e = launch_msc_one(P, st);
             }
         }
         for (const auto& cl : classes_) {
-            e = launch_msc(cl.second.first, cl.second.second, epoch, epoch_base);
-            if (e != cudaSuccess) return e;
+            const cudaStream_t st = next_stream();
+            if (e == cudaSuccess)
+                e = launch_msc(cl.second.first, cl.second.second, epoch, epoch_base, st);
         }
+        joinable_ = n_aux_ > 0;
         return e;
     }
 
@@ -890,10 +1200,17 @@ private:
             e = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
             if (e != cudaSuccess) return cuda_fail(e, "cudaStreamBeginCapture (batch)");
             cudaError_t le = cudaSuccess;
+            forked_ = false;  // the class streams join the capture, each a branch of the graph
             for (long long k = 0; k < 2 * chunk_sweeps_ && le == cudaSuccess; ++k)
                 le = launch_epoch(k, d_epoch_);
+            const int jrc = le == cudaSuccess ? join() : ISING_OK;
+            joinable_ = false;
             cudaGraph_t graph = nullptr;
             e = cudaStreamEndCapture(stream_, &graph);
+            if (jrc != ISING_OK) {
+                if (graph) cudaGraphDestroy(graph);
+                return jrc;
+            }
             if (le != cudaSuccess || e != cudaSuccess) {
                 if (graph) cudaGraphDestroy(graph);
                 return cuda_fail(le != cudaSuccess ? le : e, "batch graph capture");
@@ -909,6 +1226,7 @@ private:
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaGraphLaunch(chunk_exec_, stream_);
         if (e != cudaSuccess) return cuda_fail(e, "batch graph launch");
+        forked_ = false;  // the class streams have yet to wait for the chunk
         epoch_ += 2 * chunk_sweeps_;
         return ISING_OK;
     }
@@ -1119,7 +1437,17 @@ private:
     BatchItem* d_items_ = nullptr;
     size_t lats_cap_ = 0, items_cap_ = 0;
     std::vector<std::pair<KernelClass, std::pair<int, int>>> classes_;  // msc work items
-    std::vector<std::pair<KernelClass, std::vector<Int8Launch>>> int8_launches_;
+    std::vector<Int8Class> int8_launches_;
+    std::vector<MscLaunch> msc_one_;  // the msc class, one word per thread
+    struct Aux {
+        cudaStream_t stream = nullptr;
+        cudaEvent_t event = nullptr;
+    };
+    std::vector<Aux> aux_;           // class streams
+    size_t n_aux_ = 0;               // class streams in use (0: all on stream_)
+    cudaEvent_t fork_event_ = nullptr;
+    bool forked_ = false;            // the class streams have waited for stream_
+    bool joinable_ = false;          // stream_ has yet to wait for the class streams
     std::vector<cudaEvent_t> epoch_events_, free_events_;
     std::map<const void*, int> occupancy_;
     std::deque<std::pair<cudaEvent_t, long long>> inflight_;  // (event, epoch recorded at)
