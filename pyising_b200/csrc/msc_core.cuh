@@ -132,20 +132,26 @@ struct QueueSlots {
     u64 res[kQueueCap + 1];
 };
 
-// Threshold bit masks of the even and odd level of each level pair: (t4e, t8e, t4o, t8o).
+// The threshold bit that a lane compares with at one level is the bit of thr4 where it has one
+// anti-aligned neighbour (a1) and the bit of thr8 where it has none: 0, ~0, a1 or ~a1 over a word,
+// which is a1 * d + t modulo 2^32 with (d, t) = (0, 0), (0, -1), (1, 0) or (-1, -1).  So the mask
+// costs a multiply-add, on the multiplier pipe, instead of a logic operation with two uniform
+// masks: the logic pipe is what bounds these kernels.
+// Both levels of a level pair: (d, t) of the even level, (d, t) of the odd one.
 __device__ __forceinline__ uint4 level_masks(u32 thr4, u32 thr8, u32 lp)
 {
     const u32 se = 31u - 2u * lp, so = se - 1u;
-    return make_uint4(((thr4 >> se) & 1u) ? ~0u : 0u, ((thr8 >> se) & 1u) ? ~0u : 0u,
-                      ((thr4 >> so) & 1u) ? ~0u : 0u, ((thr8 >> so) & 1u) ? ~0u : 0u);
+    const u32 e4 = (thr4 >> se) & 1u, e8 = (thr8 >> se) & 1u;
+    const u32 o4 = (thr4 >> so) & 1u, o8 = (thr8 >> so) & 1u;
+    return make_uint4(e4 - e8, 0u - e8, o4 - o8, 0u - o8);
 }
 
-// One bit level on 32 lanes: tm selects each lane's threshold bit (thr4 for lanes with one
-// anti-aligned neighbour, thr8 for none); an undecided lane is decided when its random bit
-// differs from tm, and accepted (flipped) when that bit is 0 and tm is 1.
-__device__ __forceinline__ void level32(u32 r, u32 t4m, u32 t8m, u32 a1, u32& und, u32& res)
+__device__ __forceinline__ u32 level_mask(u32 a1, u32 d, u32 t) { return a1 * d + t; }
+
+// One bit level on 32 lanes: tm holds each lane's threshold bit; an undecided lane is decided
+// when its random bit differs from tm, and accepted (flipped) when that bit is 0 and tm is 1.
+__device__ __forceinline__ void level32(u32 r, u32 tm, u32& und, u32& res)
 {
-    const u32 tm = (a1 & t4m) | (~a1 & t8m);
     res ^= und & ~r & tm;
     und &= ~(r ^ tm);
 }
@@ -153,18 +159,17 @@ __device__ __forceinline__ void level32(u32 r, u32 t4m, u32 t8m, u32 a1, u32& un
 __device__ __forceinline__ void call_levels(const u32x4& r, const uint4& m, u32 a1l, u32 a1h,
                                             u32& undl, u32& undh, u32& resl, u32& resh)
 {
-    level32(r.x, m.x, m.y, a1l, undl, resl);  // even level: r0 | r1 << 32
-    level32(r.y, m.x, m.y, a1h, undh, resh);
-    level32(r.z, m.z, m.w, a1l, undl, resl);  // odd level: r2 | r3 << 32
-    level32(r.w, m.z, m.w, a1h, undh, resh);
+    level32(r.x, level_mask(a1l, m.x, m.y), undl, resl);  // even level: r0 | r1 << 32
+    level32(r.y, level_mask(a1h, m.x, m.y), undh, resh);
+    level32(r.z, level_mask(a1l, m.z, m.w), undl, resl);  // odd level: r2 | r3 << 32
+    level32(r.w, level_mask(a1h, m.z, m.w), undh, resh);
 }
 
 // Both levels of one Philox block on 32 lanes: the even level uses r_e, the odd one r_o.
-__device__ __forceinline__ void level_pair(u32 re, u32 ro, u32 t4e, u32 t8e, u32 t4o, u32 t8o,
-                                           u32 a1, u32& und, u32& acc)
+__device__ __forceinline__ void level_pair(u32 re, u32 ro, const uint4& m, u32 a1, u32& und,
+                                           u32& acc)
 {
-    const u32 tme = (a1 & t4e) | (~a1 & t8e);
-    const u32 tmo = (a1 & t4o) | (~a1 & t8o);
+    const u32 tme = level_mask(a1, m.x, m.y), tmo = level_mask(a1, m.z, m.w);
     const u32 ae = und & ~re & tme;       // decided at the even level, accepted
     const u32 u1 = und & ~(re ^ tme);     // still undecided after it
     const u32 ao = u1 & ~ro & tmo;
@@ -175,8 +180,8 @@ __device__ __forceinline__ void level_pair(u32 re, u32 ro, u32 t4e, u32 t8e, u32
 __device__ __forceinline__ void block_levels(const u32x4& r, const uint4& m, u32 a1l, u32 a1h,
                                              u32& undl, u32& undh, u32& accl, u32& acch)
 {
-    level_pair(r.x, r.z, m.x, m.y, m.z, m.w, a1l, undl, accl);  // r0 | r1 << 32, r2 | r3 << 32
-    level_pair(r.y, r.w, m.x, m.y, m.z, m.w, a1h, undh, acch);
+    level_pair(r.x, r.z, m, a1l, undl, accl);  // r0 | r1 << 32, r2 | r3 << 32
+    level_pair(r.y, r.w, m, a1h, undh, acch);
 }
 
 // Where a lattice piece sits in a bigger lattice (slab decomposition): the Philox word index is
@@ -239,8 +244,7 @@ struct HalfBlock {
 
 __device__ __forceinline__ HalfBlock half_block(u32 re, u32 ro, const uint4& m, u32 a1)
 {
-    const u32 tme = (a1 & m.x) | (~a1 & m.y);
-    const u32 tmo = (a1 & m.z) | (~a1 & m.w);
+    const u32 tme = level_mask(a1, m.x, m.y), tmo = level_mask(a1, m.z, m.w);
     const u32 eq = ~(re ^ tme);
     HalfBlock h;
     h.lt = (~re & tme) | (eq & ~ro & tmo);
@@ -422,13 +426,18 @@ __device__ __forceinline__ void msc_queue_range(const MscHalf& p, long long begi
 // of one 32-word column strip, lane l owning word x0 + l of every row.  The opposite colour's
 // rows y - 1, y, y + 1 slide through registers (one new row per step), so a word costs three
 // loads (its own word, the opposite colour's next row, the horizontal neighbour word) instead
-// of five, and the row parity, the row index and the wrap of the vertical neighbours are
-// warp-uniform.  The bit-sliced count takes seven operations per 32-bit half: with
-// x_k = o ^ n_k, x1 ^ x2 = n1 ^ n2 and x1 & x2 = (o ^ n1) & (o ^ n2), so the pair sums need
-// no x_k.  The lazy comparison handles both levels of a Philox block together (seven
-// operations per half).  Words still undecided after the intake go to the warp's stack as in
-// the range schedule.  Random numbers, levels and their order are the reference's, so the
-// results are identical.
+// of five, and the row index and the wrap of the vertical neighbours are warp-uniform.  The
+// bit-sliced count takes seven operations per 32-bit half: with x_k = o ^ n_k, x1 ^ x2 = n1 ^ n2
+// and x1 & x2 = (o ^ n1) & (o ^ n2), so the pair sums need no x_k.  Words still undecided after
+// the intake go to the warp's stack as in the range schedule.  Random numbers, levels and their
+// order are the reference's, so the results are identical.
+//
+// The kernel is bound by the logic pipe (two cycles per warp and SM quarter for each logic,
+// compare or shift instruction and for each wide multiply of the random numbers): 231 such slots
+// per word, 258 with the level masks as logic operations, the undecided lanes carried down the
+// levels and either row parity in one loop.  16384^2 on one B200, flips/ns: 3714 before, 3838 with
+// the masks as multiply-adds, 4053 with even bands of a fixed parity and the levels from the last
+// to the first; 8192^2 2837 -> 3015.  Blocks of 4 to 10 warps (3237-3958) were slower.
 
 // Pair sums of two anti-aligned flags: s = exactly one, c = both.
 struct HalfSlices {
@@ -447,9 +456,8 @@ __device__ __forceinline__ HalfSlices slice_half(u32 o, u32 n1, u32 n2, u32 n3, 
 }
 
 // The warp walks its band two rows per step: each lane takes word x of rows y and y + 1, so
-// eight Philox chains are in flight at intake and the per-step loop, ballot and stack
-// bookkeeping are shared by two words.  The stack takes up to 64 entries per intake, so it holds
-// kPop + 64.  The Philox products are separate high and low multiplies and the intake's level
+// the per-step loop, ballot and stack bookkeeping are shared by two words.  The stack takes up
+// to 64 entries per intake, so it holds kPop + 64.  The Philox products are separate high and low multiplies and the intake's level
 // masks come from the block's shared table: measured faster here (16384^2: 3610 flips/ns
 // against 3260 for one row per step with the products as wide multiplies and the masks derived
 // in uniform registers).
@@ -504,58 +512,65 @@ __device__ __forceinline__ void strip_pop(const MscHalf& p, StripSlots& q, int& 
     __syncwarp();
 }
 
-// The warp updates rows [y0, y1) of strip `strip` (words 32 strip .. 32 strip + 31 of a row).
+// Two levels on top of what the less significant ones decide: lt = accepted, eq = undecided, over
+// the lanes as if none were decided before.  Going from the last block to the first this takes one
+// operation less per block and half than carrying the undecided lanes down (level_pair).
+__device__ __forceinline__ void level_pair_up(u32 re, u32 ro, const uint4& m, u32 a1, u32& eq,
+                                              u32& lt)
+{
+    const u32 tme = level_mask(a1, m.x, m.y), tmo = level_mask(a1, m.z, m.w);
+    lt = (~ro & tmo) | (~(ro ^ tmo) & lt);
+    eq &= ~(ro ^ tmo);
+    lt = (~re & tme) | (~(re ^ tme) & lt);
+    eq &= ~(re ^ tme);
+}
+
+// The warp updates rows [y0, y1) of strip `strip` (words 32 strip .. 32 strip + 31 of a row), an
+// even number of rows.
 // SLAB: the lattice is a slab of a bigger one (SlabOffset): Philox word indices are so.w0 + the
 // local index, row parities those of the global rows, and rows -1 and `rows` of the opposite
 // colour are read from so.lo and so.hi instead of wrapping.
-template <int K, bool SLAB = false>
-__device__ __forceinline__ void msc_strip_band(const MscHalf& p, int strip, int y0, int y1,
-                                               StripSlots& q, const uint4* lvmask,
-                                               const SlabOffset& so = {0, 0, nullptr, nullptr})
+// ODD: the parity of row y0 (+ colour), which every pair of rows starts with.
+template <int K, bool SLAB, bool ODD>
+__device__ __forceinline__ void msc_strip_pairs(const MscHalf& p, int strip, int y0, int y1,
+                                                StripSlots& q, const uint4* lvmask,
+                                                const SlabOffset& so)
 {
     const int lane = threadIdx.x & 31;
-    const u32 lt = (1u << lane) - 1u;
+    const u32 lt_mask = (1u << lane) - 1u;
     const int nw = p.nw, rows = p.rows;
     const int x = strip * 32 + lane;
     const int xr = x + 1 == nw ? 0 : x + 1, xl = x == 0 ? nw - 1 : x - 1;
-    const u64* other = p.other;
     const u32 wg = SLAB ? (u32)so.w0 : 0u;
-    const int odd0 = ((SLAB ? so.par0 : 0) + (int)p.color) & 1;  // parity of local row 0
-    // opposite-colour row r, r in [-1, rows]
-    auto orow = [&](int r) -> const u64* {
-        if constexpr (SLAB) {
-            if (r < 0) return so.lo;
-            if (r >= rows) return so.hi;
-        } else {
-            r = r < 0 ? rows - 1 : (r >= rows ? 0 : r);
-        }
-        return other + (long long)r * nw;
-    };
-    u64 up = __ldg(orow(y0 - 1) + x);
-    u64 c = __ldg(orow(y0) + x);
-    u64 f_o0 = 0, f_o1 = 0, f_d1 = 0, f_d2 = 0, f_s0 = 0, f_s1 = 0;
+    // where the words of rows y and y + 1 are, from the current row pair
+    const int side0 = (ODD ? xr : xl) - x, side1 = (ODD ? xl : xr) - x;
+    const u64* oc = p.other + (long long)y0 * nw + x;  // opposite colour, row y
+    u64* own = p.own + (long long)y0 * nw + x;
+    const u64* after = (SLAB ? so.hi : p.other) + x;   // row `rows` of the opposite colour
+    u64 up = __ldg(y0 == 0 ? (SLAB ? so.lo : p.other + (long long)(rows - 1) * nw) + x : oc - nw);
+    u64 c = __ldg(oc);
+    u64 f_o0, f_o1, f_d1, f_d2, f_s0, f_s1;
     auto fetch = [&](int y) {
-        f_o0 = p.own[(long long)y * nw + x];
-        f_d1 = __ldg(orow(y + 1) + x);
-        f_s0 = __ldg(orow(y) + (((y + odd0) & 1) ? xr : xl));
-        if (y + 1 < y1) {
-            f_o1 = p.own[(long long)(y + 1) * nw + x];
-            f_d2 = __ldg(orow(y + 2) + x);
-            f_s1 = __ldg(orow(y + 1) + (((y + 1 + odd0) & 1) ? xr : xl));
-        }
+        f_o0 = own[0];
+        f_o1 = own[nw];
+        f_d1 = __ldg(oc + nw);
+        f_d2 = __ldg(y + 2 == rows ? after : oc + 2 * (long long)nw);
+        f_s0 = __ldg(oc + side0);
+        f_s1 = __ldg(oc + (nw + side1));
     };
     int y = y0;
-    if (y < y1) fetch(y);
+    fetch(y);
+    u32 wa = (u32)((long long)y0 * nw + x);
     int n = 0;
     while (true) {
         if (n < kPop && y < y1) {
-            const bool two = y + 1 < y1;
             const u64 o0 = f_o0, o1 = f_o1, d1 = f_d1, d2 = f_d2, s0 = f_s0, s1 = f_s1;
-            const bool odd = ((y + odd0) & 1) != 0;  // row y; row y + 1 has the other parity
-            const u64 hz0 = odd ? ((c >> 1) | (s0 << 63)) : ((c << 1) | (s0 >> 63));
-            const u64 hz1 = odd ? ((d1 << 1) | (s1 >> 63)) : ((d1 >> 1) | (s1 << 63));
-            const int yc = y;
-            y += two ? 2 : 1;
+            const u64 hz0 = ODD ? ((c >> 1) | (s0 << 63)) : ((c << 1) | (s0 >> 63));
+            const u64 hz1 = ODD ? ((d1 << 1) | (s1 >> 63)) : ((d1 >> 1) | (s1 << 63));
+            u64* dst = own;
+            y += 2;
+            own += 2 * (long long)nw;
+            oc += 2 * (long long)nw;
             if (y < y1) fetch(y);
             const HalfSlices al = slice_half((u32)o0, (u32)c, (u32)hz0, (u32)up, (u32)d1);
             const HalfSlices ah = slice_half((u32)(o0 >> 32), (u32)(c >> 32), (u32)(hz0 >> 32),
@@ -563,34 +578,40 @@ __device__ __forceinline__ void msc_strip_band(const MscHalf& p, int strip, int 
             const HalfSlices bl = slice_half((u32)o1, (u32)d1, (u32)hz1, (u32)c, (u32)d2);
             const HalfSlices bh = slice_half((u32)(o1 >> 32), (u32)(d1 >> 32), (u32)(hz1 >> 32),
                                              (u32)(c >> 32), (u32)(d2 >> 32));
-            up = two ? d1 : c;
-            c = two ? d2 : d1;
-            u32 ual = ~al.a2, uah = ~ah.a2, aal = 0, aah = 0;
-            u32 ubl = ~bl.a2, ubh = ~bh.a2, abl = 0, abh = 0;
-            const u32 wa = (u32)((long long)yc * nw + x), wb = wa + (u32)nw;
+            up = d1;
+            c = d2;
+            const u32 wb = wa + (u32)nw;
+            u32 ual = ~0u, uah = ~0u, ubl = ~0u, ubh = ~0u;
+            u32 aal = 0, aah = 0, abl = 0, abh = 0;
 #pragma unroll
-            for (int b = 0; b < K; ++b) {
+            for (int b = K - 1; b >= 0; --b) {
                 const uint4 m = lvmask[b];
                 const u32x4 ra =
                     philox4x32_10<true>(wg + wa, p.t, p.color, 1u + (u32)b, p.k0, p.k1);
                 const u32x4 rb =
                     philox4x32_10<true>(wg + wb, p.t, p.color, 1u + (u32)b, p.k0, p.k1);
-                block_levels(ra, m, al.a1, ah.a1, ual, uah, aal, aah);
-                block_levels(rb, m, bl.a1, bh.a1, ubl, ubh, abl, abh);
+                level_pair_up(ra.x, ra.z, m, al.a1, ual, aal);  // r0 | r1 << 32, r2 | r3 << 32
+                level_pair_up(ra.y, ra.w, m, ah.a1, uah, aah);
+                level_pair_up(rb.x, rb.z, m, bl.a1, ubl, abl);
+                level_pair_up(rb.y, rb.w, m, bh.a1, ubh, abh);
             }
-            const u32 ral = (u32)o0 ^ al.a2 ^ aal, rah = (u32)(o0 >> 32) ^ ah.a2 ^ aah;
-            const u32 rbl = (u32)o1 ^ bl.a2 ^ abl, rbh = (u32)(o1 >> 32) ^ bh.a2 ^ abh;
-            const bool ka = (ual | uah) != 0, kb = two && (ubl | ubh) != 0;
+            ual &= ~al.a2;
+            uah &= ~ah.a2;
+            ubl &= ~bl.a2;
+            ubh &= ~bh.a2;
+            const u32 ral = (u32)o0 ^ (al.a2 | aal), rah = (u32)(o0 >> 32) ^ (ah.a2 | aah);
+            const u32 rbl = (u32)o1 ^ (bl.a2 | abl), rbh = (u32)(o1 >> 32) ^ (bh.a2 | abh);
+            const bool ka = (ual | uah) != 0, kb = (ubl | ubh) != 0;
             // every word is stored, decided or not: an undecided word's entry ends with the
             // store of its final value, and nothing else reads this colour during the
             // half-sweep (measured 0.6-0.8% faster than storing only the decided words here; in
             // the word-range walker 0.5% slower, so that one keeps the predicated store)
-            p.own[wa] = (u64)ral | ((u64)rah << 32);
-            if (two) p.own[wb] = (u64)rbl | ((u64)rbh << 32);
+            dst[0] = (u64)ral | ((u64)rah << 32);
+            dst[nw] = (u64)rbl | ((u64)rbh << 32);
             const u32 kma = __ballot_sync(0xFFFFFFFFu, ka);
             const u32 kmb = __ballot_sync(0xFFFFFFFFu, kb);
             {
-                const int pos = ka ? n + __popc(kma & lt) : kStripCap;
+                const int pos = ka ? n + __popc(kma & lt_mask) : kStripCap;
                 q.idx[pos] = wa;
                 q.lp[pos] = (u32)K;
                 q.a1[pos] = (u64)al.a1 | ((u64)ah.a1 << 32);
@@ -599,7 +620,7 @@ __device__ __forceinline__ void msc_strip_band(const MscHalf& p, int strip, int 
             }
             n += __popc(kma);
             {
-                const int pos = kb ? n + __popc(kmb & lt) : kStripCap;
+                const int pos = kb ? n + __popc(kmb & lt_mask) : kStripCap;
                 q.idx[pos] = wb;
                 q.lp[pos] = (u32)K;
                 q.a1[pos] = (u64)bl.a1 | ((u64)bh.a1 << 32);
@@ -607,6 +628,7 @@ __device__ __forceinline__ void msc_strip_band(const MscHalf& p, int strip, int 
                 q.res[pos] = (u64)rbl | ((u64)rbh << 32);
             }
             n += __popc(kmb);
+            wa += 2u * (u32)nw;
             __syncwarp();
         } else if (y >= y1 && n <= 32) {
             if (n > 0) stack_drain(p, q, n, lvmask, wg);
@@ -614,6 +636,39 @@ __device__ __forceinline__ void msc_strip_band(const MscHalf& p, int strip, int 
         } else {
             strip_pop(p, q, n, lvmask, wg);
         }
+    }
+}
+
+// Rows [y0, y1) of a strip: pairs of rows on the work stack, and a last single row (bands are even
+// but where a slab's own rows are not) a word per lane.
+template <int K, bool SLAB = false>
+__device__ __forceinline__ void msc_strip_band(const MscHalf& p, int strip, int y0, int y1,
+                                               StripSlots& q, const uint4* lvmask,
+                                               const SlabOffset& so = {0, 0, nullptr, nullptr})
+{
+    const int ye = y1 - ((y1 - y0) & 1);
+    if (ye > y0) {
+        if ((y0 + (SLAB ? so.par0 : 0) + (int)p.color) & 1)
+            msc_strip_pairs<K, SLAB, true>(p, strip, y0, ye, q, lvmask, so);
+        else
+            msc_strip_pairs<K, SLAB, false>(p, strip, y0, ye, q, lvmask, so);
+    }
+    if (ye < y1) {
+        const long long w = (long long)ye * p.nw + strip * 32 + (int)(threadIdx.x & 31);
+        IntakeLoads L;
+        intake_load<SLAB>(p, w, true, p.nw, -1, L, so);
+        const bool par = ((SLAB ? L.y + so.par0 : L.y) + (int)p.color) & 1;
+        const u64 hz = par ? ((L.c >> 1) | (L.side << 63)) : ((L.c << 1) | (L.side >> 63));
+        const HalfSlices al = slice_half((u32)L.o, (u32)L.c, (u32)hz, (u32)L.up, (u32)L.dn);
+        const HalfSlices ah = slice_half((u32)(L.o >> 32), (u32)(L.c >> 32), (u32)(hz >> 32),
+                                         (u32)(L.up >> 32), (u32)(L.dn >> 32));
+        u32 ul = ~al.a2, uh = ~ah.a2, accl = 0, acch = 0;
+        for (u32 lp = 0; lp < 16u && (ul | uh) != 0; ++lp) {
+            const u32x4 r = philox4x32_10<true>((SLAB ? (u32)so.w0 : 0u) + (u32)w, p.t, p.color,
+                                                1u + lp, p.k0, p.k1);
+            block_levels(r, lvmask[lp], al.a1, ah.a1, ul, uh, accl, acch);
+        }
+        p.own[w] = L.o ^ ((u64)(al.a2 | accl) | ((u64)(ah.a2 | acch) << 32));
     }
 }
 

@@ -145,7 +145,8 @@ static cudaError_t launch_strip(const MscHalf& p, int sm_count, int waves, cudaS
     const long long warps = (long long)(sm_count > 0 ? sm_count : 1) *
                             strip_blocks_per_sm<MEAS, K, MINB>() * kQueueWarps * (waves > 0 ? waves : 1);
     long long band = (units + warps - 1) / warps;
-    if (band < 1) band = 1;
+    band += band & 1;  // pairs of rows
+    if (band < 2) band = 2;
     const long long nwarps = (long long)strips * ((p.rows + band - 1) / band);
     const unsigned blocks = (unsigned)((nwarps + kQueueWarps - 1) / kQueueWarps);
     return launch_pdl(msc_strip_kernel<MEAS, K, MINB>, dim3(blocks), dim3(kQueueWarps * 32), st, p,

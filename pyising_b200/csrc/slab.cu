@@ -250,7 +250,8 @@ static cudaError_t launch_msc_slab_strip(const MscHalf& p, const SlabOffset& so,
     const long long units = (long long)an * strips;
     const long long warps = (long long)sm_count * blocks_per_sm * kSlabStripWarps;
     long long band = (units + warps - 1) / warps;
-    if (band < 1) band = 1;
+    band += band & 1;  // pairs of rows
+    if (band < 2) band = 2;
     const long long nwarps = (long long)strips * ((an + band - 1) / band);
     const unsigned blocks = (unsigned)((nwarps + kSlabStripWarps - 1) / kSlabStripWarps);
     return launch_pdl(msc_slab_strip_kernel, dim3(blocks), dim3(kSlabStripWarps * 32), st, p, so,
