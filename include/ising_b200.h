@@ -117,7 +117,7 @@ int ising_half_sweep(ising_sim* h, int color, uint64_t t);
  *   ISING_SCHEDULE_GRAPHS     replayed CUDA graphs of whole chunks of sweeps;
  *   ISING_SCHEDULE_PERSISTENT one cooperative launch for all sweeps (2D int8; others fall back):
  *                             bands of rows wait only for their neighbours, every wait bounded;
- *   ISING_SCHEDULE_TEMPORAL   graphs whose launches each run several half-sweeps on
+ *   ISING_SCHEDULE_TEMPORAL   launches that each run several half-sweeps on
  *                             shared-memory tiles with recomputed halos (2D lattices whose
  *                             rows fit; others fall back).
  * All schedules give identical results.  test_mute_band >= 0 makes that band of a persistent

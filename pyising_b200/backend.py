@@ -134,9 +134,10 @@ class _B200Simulation(IsingSimulation):
     def set_schedule(self, schedule: str = "auto", test_mute_band: int = -1) -> None:
         """How sweeps are issued: ``"auto"``, ``"launches"`` (one kernel per half-sweep),
         ``"graphs"`` (replayed CUDA graphs), ``"persistent"`` (one cooperative launch for all
-        sweeps; 2D int8) or ``"temporal"`` (graphs of launches that each run several half-sweeps
-        on shared-memory tiles; 2D lattices).  Results are identical.  ``test_mute_band`` >= 0 is a test hook that
-        makes one band of a persistent run stop publishing, so the run reports a time-out."""
+        sweeps; 2D int8) or ``"temporal"`` (launches that each run several half-sweeps on
+        shared-memory tiles; 2D lattices).  Results are identical.  ``test_mute_band`` >= 0 is a
+        test hook that makes one band of a persistent run stop publishing, so the run reports a
+        time-out."""
         check(lib().ising_set_schedule(self._h, self.SCHEDULES[schedule], int(test_mute_band)),
               "set_schedule")
 

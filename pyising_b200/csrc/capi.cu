@@ -201,14 +201,7 @@ static int chunk_graph(ising_sim* h, int64_t G, bool measured, cudaGraphExec_t* 
     cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamBeginCapture");
     int rc = ISING_OK;
-    int64_t s = 0;
-    if (use_temporal(h)) {
-        const cudaError_t le = launch_temporal_run(
-            h, 0u, G, measured ? (unsigned long long*)h->d_series : nullptr, ctl);
-        if (le != cudaSuccess) rc = cuda_fail(le, "temporal half-sweeps");
-        s = G;
-    }
-    for (; s < G && rc == ISING_OK;) {
+    for (int64_t s = 0; s < G && rc == ISING_OK;) {
         unsigned long long* m =
             (measured && s == G - 1) ? (unsigned long long*)h->d_series : nullptr;
         rc = half_sweep(h, 0, (u32)s, nullptr, nullptr, ctl);
@@ -701,9 +694,18 @@ int ising_sweep(ising_sim* h, uint64_t t0, int64_t n_sweeps, int64_t measure_eve
         TRY_CUDA(cudaMemsetAsync(h->d_series, 0, (size_t)n_meas * 2 * sizeof(long long),
                                  h->stream));
     }
-    if (use_temporal(h)) {  // before any graph capture
-        int rc = temporal_scratch(h);
-        if (rc != ISING_OK) return rc;
+    // The tiles need their second pair of arrays.  A stream that is being captured cannot allocate
+    // it for later use, and without memory for it the automatic schedule does without the tiles.
+    bool tiles = use_temporal(h);
+    if (tiles && !(h->tb_scratch[0] && h->tb_scratch[1])) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        TRY_CUDA(cudaStreamIsCapturing(h->stream, &capture));
+        tiles = capture == cudaStreamCaptureStatusNone;
+        if (tiles) {
+            const int rc = temporal_scratch(h);
+            if (rc != ISING_OK && h->schedule == ISING_SCHEDULE_TEMPORAL) return rc;
+            tiles = rc == ISING_OK;
+        }
     }
     int64_t k = 0, s0 = 0;
     // Small 2D int8 lattices: all sweeps in one persistent cooperative launch.
@@ -739,10 +741,28 @@ int ising_sweep(ising_sim* h, uint64_t t0, int64_t n_sweeps, int64_t measure_eve
         }
         if (rc != ISING_ERR_STATE) return rc;  // ISING_ERR_STATE: not resident, fall back
     }
+    // Tiles are launched directly, one run up to each measured sweep: a launch holds several
+    // half-sweeps, longer than the host takes to issue the next, while a graph per run ends with a
+    // kernel that advances its counters and cannot overlap the tiles (measured on one B200: the
+    // 1152^2 msc lattice measured every 10 sweeps 3.1 us a sweep with graphs, 2.7 without; five
+    // temperatures of a 128^2 lattice 1731 and 1002 us, mostly graph captures).
+    while (tiles && s0 < n_sweeps) {
+        int64_t run = n_sweeps - s0;
+        bool meas = false;
+        if (measure_every > 0 && measure_every - s0 % measure_every <= run) {
+            run = measure_every - s0 % measure_every;
+            meas = true;
+        }
+        TRY_CUDA(launch_temporal_run(h, (u32)(t0 + (uint64_t)s0), run,
+                                     meas ? (unsigned long long*)(h->d_series + 2 * k) : nullptr));
+        s0 += run;
+        if (meas) ++k;
+    }
     // Whole chunks of G sweeps replay one captured graph (G = the measurement interval, so each
     // chunk ends with its measurement); the rest is launched directly.
     const int64_t G = measure_every > 0 ? measure_every : h->graph_chunk;
-    if (h->schedule != ISING_SCHEDULE_LAUNCHES && G <= kGraphChunkMax && n_sweeps >= 2 * G) {
+    if (h->schedule != ISING_SCHEDULE_LAUNCHES && G <= kGraphChunkMax &&
+        n_sweeps - s0 >= 2 * G) {
         cudaGraphExec_t exec = nullptr;
         int rc = chunk_graph(h, G, measure_every > 0, &exec);
         if (rc != ISING_OK) return rc;
@@ -763,19 +783,6 @@ int ising_sweep(ising_sim* h, uint64_t t0, int64_t n_sweeps, int64_t measure_eve
             TRY_CUDA(cudaGraphLaunch(rexec, h->stream));
             s0 = n_sweeps;
         }
-    }
-    while (use_temporal(h) && s0 < n_sweeps) {  // up to the next measured sweep, or the end
-        int64_t run = n_sweeps - s0;
-        bool meas = false;
-        if (measure_every > 0 && measure_every - s0 % measure_every <= run) {
-            run = measure_every - s0 % measure_every;
-            meas = true;
-        }
-        TRY_CUDA(launch_temporal_run(h, (u32)(t0 + (uint64_t)s0), run,
-                                     meas ? (unsigned long long*)(h->d_series + 2 * k) : nullptr,
-                                     nullptr));
-        s0 += run;
-        if (meas) ++k;
     }
     for (int64_t s = s0; s < n_sweeps; ++s) {
         const u32 t = (u32)(t0 + (uint64_t)s);

@@ -80,7 +80,7 @@ int temporal_scratch(ising_sim* h);
 // `sweeps` sweeps from sweep t on the temporal schedule, (M, E) of the last one into meas (unless
 // null); the lattice ends in the handle's arrays.
 cudaError_t launch_temporal_run(const ising_sim* h, u32 t, int64_t sweeps,
-                                unsigned long long* meas, const unsigned long long* ctl);
+                                unsigned long long* meas);
 int run_persistent_int8(ising_sim* h, uint64_t t0, int64_t n_sweeps, int64_t measure_every,
                         unsigned long long* series, unsigned int* flags, int* err, int mute_band);
 int selftest_bounded_wait(int device, int* timed_out);

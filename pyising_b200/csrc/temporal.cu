@@ -77,7 +77,6 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     __shared__ u32 rt[kLookupWords];                // the lookup table of the decisions
     Int8Half p = p_in;
     if (threadIdx.x == 0) fill_lookup<2, RULE>(rt, p.table);
-    resolve_ctl(p);  // written between graph replays only (see int8_one_kernel)
     const int ly = p.ly, pitch = p.pitch, cpr = p.cpr;
     const Tile T(run, ly);
     const int stride = T.rows * pitch;
@@ -179,7 +178,6 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     __shared__ uint4 lvmask[16];
     MscHalf p = p_in;
     if (threadIdx.x < 16) lvmask[threadIdx.x] = level_masks(p.thr4, p.thr8, threadIdx.x);
-    resolve_ctl(p);
     const int ly = p.rows, nw = p.nw;
     const Tile T(run, ly);
     const int stride = T.rows * nw;
@@ -402,8 +400,7 @@ static cudaError_t launch_int8_tile(int rule, const Int8Half& p, const TileRun& 
 // One launch: half-sweeps h0 .. h0 + depth - 1 from sweep t, from the handle's arrays into its
 // scratch pair (to_scratch) or back; meas: the (M, E) accumulators of its last half-sweep.
 static cudaError_t launch_tiles(const ising_sim* h, u32 t, int h0, int depth, int band,
-                                unsigned long long* meas, const unsigned long long* ctl,
-                                bool to_scratch)
+                                unsigned long long* meas, bool to_scratch)
 {
     TileRun run{h0, depth, band, 0};
     const unsigned blocks = (unsigned)((h->ly + band - 1) / band);
@@ -422,7 +419,6 @@ static cudaError_t launch_tiles(const ising_sim* h, u32 t, int h0, int depth, in
         p.thr4 = h->table[3];
         p.thr8 = h->table[4];
         p.meas = meas;
-        p.ctl = ctl;
         run.items_magic = fast_div_magic((u32)p.nw, rows * p.nw);
         const u64 *i0 = (const u64*)in[0], *i1 = (const u64*)in[1];
         u64 *o0 = (u64*)out[0], *o1 = (u64*)out[1];
@@ -462,7 +458,6 @@ static cudaError_t launch_tiles(const ising_sim* h, u32 t, int h0, int depth, in
     p.k1 = (u32)(h->seed >> 32);
     for (int i = 0; i < 7; ++i) p.table[i] = h->table[i];
     p.meas = meas;
-    p.ctl = ctl;
     run.items_magic = fast_div_magic((u32)p.cpr, rows * p.cpr);
     const int8_t *i0 = (const int8_t*)in[0], *i1 = (const int8_t*)in[1];
     int8_t *o0 = (int8_t*)out[0], *o1 = (int8_t*)out[1];
@@ -488,7 +483,7 @@ int temporal_scratch(ising_sim* h)
 // launches of about the same depth, alternating between the handle's arrays and the scratch pair,
 // so that the lattice ends in the handle's arrays.
 cudaError_t launch_temporal_run(const ising_sim* h, u32 t, int64_t sweeps,
-                                unsigned long long* meas, const unsigned long long* ctl)
+                                unsigned long long* meas)
 {
     int band = 0, depth = 0;
     tile_shape(h, &band, &depth);
@@ -500,7 +495,7 @@ cudaError_t launch_temporal_run(const ising_sim* h, u32 t, int64_t sweeps,
         const bool last = next == halves;
         const cudaError_t e =
             launch_tiles(h, t + (u32)(done >> 1), (int)(done & 1), (int)(next - done), band,
-                         last ? meas : nullptr, ctl, (i & 1) == 0);
+                         last ? meas : nullptr, (i & 1) == 0);
         if (e != cudaSuccess) return e;
         done = next;
     }

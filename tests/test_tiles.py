@@ -55,3 +55,32 @@ def test_msc_tiles(oracle_mod, shape, beta):
         np.testing.assert_array_equal(w1, ref.w[1])
 
     run(sim, ref, final)
+
+
+def test_sweeps_into_a_captured_stream():
+    """Sweeps issued into a stream under capture: without the tiles' second arrays (a capture cannot
+    allocate them for later use) and, after a sweep outside it, with them."""
+    import torch
+
+    from pyising_b200.backend import B200MultiSpin
+
+    for warm in (False, True):
+        a = B200MultiSpin((64, 256), BETA_C_2D, seed=3, init="philox")
+        b = B200MultiSpin((64, 256), BETA_C_2D, seed=3, init="philox")
+        if warm:
+            a.sweep(2)
+            b.sweep(2)
+        a.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            a.set_stream(torch.cuda.current_stream().cuda_stream)
+            a.sweep(3)
+        a.set_stream(None)
+        graph.replay()
+        torch.cuda.synchronize()
+        b.sweep(3)
+        for x, y in zip(a.colour_arrays(), b.colour_arrays(), strict=True):
+            np.testing.assert_array_equal(x, y)
+        a.sweep(5)
+        b.sweep(5)
+        assert a.observables_int() == b.observables_int()
