@@ -382,11 +382,11 @@ int ising_destroy(ising_sim* h)
     if (h->d_series) cudaFreeAsync(h->d_series, fs);
     for (int c = 0; c < 2; ++c)
         if (h->tb_scratch[c]) cudaFreeAsync(h->tb_scratch[c], fs);
+    if (h->d_label) cudaFreeAsync(h->d_label, fs);
     if (h->h_series) host_pinned_put(h->h_series, (size_t)h->series_cap * 2 * sizeof(long long));
     if (fs) cudaStreamSynchronize(fs);
     clear_graphs(h);
     if (h->d_flags) cudaFree(h->d_flags);
-    if (h->d_label) cudaFree(h->d_label);
     if (h->own_stream_handle) cudaStreamDestroy(h->own_stream_handle);
     cudaGetLastError();
     delete h;

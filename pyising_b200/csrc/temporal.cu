@@ -469,7 +469,10 @@ int temporal_scratch(ising_sim* h)
 {
     for (int c = 0; c < 2; ++c) {
         if (h->tb_scratch[c]) continue;
-        const cudaError_t e = pool_alloc(h->device, &h->tb_scratch[c], h->colour_bytes, h->stream);
+        // on a stream that is then waited for: usable from any stream the handle is given later
+        cudaError_t e =
+            pool_alloc(h->device, &h->tb_scratch[c], h->colour_bytes, h->own_stream_handle);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(h->own_stream_handle);
         if (e != cudaSuccess) {
             cudaGetLastError();
             h->tb_scratch[c] = nullptr;
