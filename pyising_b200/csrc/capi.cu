@@ -30,6 +30,8 @@ int cuda_fail(cudaError_t e, const char* what)
     return fail(ISING_ERR_CUDA, "%s: %s (%s)", what, cudaGetErrorString(e), cudaGetErrorName(e));
 }
 
+constexpr size_t kObsBytes = 2 * sizeof(long long);
+
 // Device memory of simulation handles comes from one stream-ordered pool per device that keeps
 // up to kPoolKeep bytes of freed memory for reuse: creating and destroying many simulations
 // (a scan, a validation run, jobs one at a time) then maps no memory and synchronises nothing.
@@ -384,6 +386,7 @@ int ising_destroy(ising_sim* h)
         if (h->tb_scratch[c]) cudaFreeAsync(h->tb_scratch[c], fs);
     if (h->d_label) cudaFreeAsync(h->d_label, fs);
     if (h->h_series) host_pinned_put(h->h_series, (size_t)h->series_cap * 2 * sizeof(long long));
+    if (h->h_obs) host_pinned_put(h->h_obs, kObsBytes);
     if (fs) cudaStreamSynchronize(fs);
     clear_graphs(h);
     if (h->d_flags) cudaFree(h->d_flags);
@@ -511,20 +514,32 @@ int ising_get_lattice(ising_sim* h, int8_t* full)
     return rc;
 }
 
+// Copies the two colour arrays between the host, where rows are contiguous, and the device, where
+// they are `pitch` apart (one piece when that is the same), and waits for the copies.
+static int copy_colours(ising_sim* h, void* const dst[2], const void* const src[2],
+                        cudaMemcpyKind kind)
+{
+    TRY_CUDA(cudaSetDevice(h->device));
+    const size_t width = host_row_bytes(h), rows = (size_t)h->rows;
+    const size_t pitch = device_row_bytes(h);
+    const bool up = kind == cudaMemcpyHostToDevice;
+    for (int c = 0; c < 2; ++c) {
+        if (pitch == width)
+            TRY_CUDA(cudaMemcpyAsync(dst[c], src[c], rows * width, kind, h->stream));
+        else
+            TRY_CUDA(cudaMemcpy2DAsync(dst[c], up ? pitch : width, src[c], up ? width : pitch,
+                                       width, rows, kind, h->stream));
+    }
+    TRY_CUDA(cudaStreamSynchronize(h->stream));
+    return ISING_OK;
+}
+
 int ising_upload(ising_sim* h, const void* c0, const void* c1)
 {
     CHECK_HANDLE(h);
     if (!c0 || !c1) return fail(ISING_ERR_INVALID, "null colour array");
-    TRY_CUDA(cudaSetDevice(h->device));
-    // host rows are contiguous (width) on the host, `pitch` apart on the device
-    const size_t width = host_row_bytes(h), rows = (size_t)h->rows;
-    const size_t dp = device_row_bytes(h);
-    TRY_CUDA(cudaMemcpy2DAsync(h->c[0], dp, c0, width, width, rows, cudaMemcpyHostToDevice,
-                               h->stream));
-    TRY_CUDA(cudaMemcpy2DAsync(h->c[1], dp, c1, width, width, rows, cudaMemcpyHostToDevice,
-                               h->stream));
-    TRY_CUDA(cudaStreamSynchronize(h->stream));
-    return ISING_OK;
+    const void* src[2] = {c0, c1};
+    return copy_colours(h, h->c, src, cudaMemcpyHostToDevice);
 }
 
 int ising_download(ising_sim* h, void* c0, void* c1)
@@ -535,15 +550,8 @@ int ising_download(ising_sim* h, void* c0, void* c1)
         if (prc != ISING_OK) return prc;
     }
     if (!c0 || !c1) return fail(ISING_ERR_INVALID, "null colour array");
-    TRY_CUDA(cudaSetDevice(h->device));
-    const size_t width = host_row_bytes(h), rows = (size_t)h->rows;
-    const size_t dp = device_row_bytes(h);
-    TRY_CUDA(cudaMemcpy2DAsync(c0, width, h->c[0], dp, width, rows, cudaMemcpyDeviceToHost,
-                               h->stream));
-    TRY_CUDA(cudaMemcpy2DAsync(c1, width, h->c[1], dp, width, rows, cudaMemcpyDeviceToHost,
-                               h->stream));
-    TRY_CUDA(cudaStreamSynchronize(h->stream));
-    return ISING_OK;
+    void* dst[2] = {c0, c1};
+    return copy_colours(h, dst, h->c, cudaMemcpyDeviceToHost);
 }
 
 int ising_fill_cold(ising_sim* h)
@@ -823,14 +831,14 @@ int ising_observables(ising_sim* h, int64_t* m, int64_t* e)
     }
     if (!m || !e) return fail(ISING_ERR_INVALID, "null output pointer");
     TRY_CUDA(cudaSetDevice(h->device));
-    TRY_CUDA(cudaMemsetAsync(h->d_acc, 0, 2 * sizeof(unsigned long long), h->stream));
+    if (!h->h_obs) TRY_CUDA(host_pinned_get((void**)&h->h_obs, kObsBytes));
+    TRY_CUDA(cudaMemsetAsync(h->d_acc, 0, kObsBytes, h->stream));
     int rc = observe(h, h->d_acc);
     if (rc != ISING_OK) return rc;
-    long long out[2];
-    TRY_CUDA(cudaMemcpyAsync(out, h->d_acc, sizeof out, cudaMemcpyDeviceToHost, h->stream));
+    TRY_CUDA(cudaMemcpyAsync(h->h_obs, h->d_acc, kObsBytes, cudaMemcpyDeviceToHost, h->stream));
     TRY_CUDA(cudaStreamSynchronize(h->stream));
-    *m = out[0];
-    *e = out[1];
+    *m = h->h_obs[0];
+    *e = h->h_obs[1];
     return ISING_OK;
 }
 

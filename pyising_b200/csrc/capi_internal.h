@@ -33,6 +33,7 @@ struct ising_sim {
     unsigned long long* d_acc = nullptr;  // [0,1] observables, [2,3] msc call statistics
     long long* d_series = nullptr;        // (M, E) pairs of one ising_sweep call
     long long* h_series = nullptr;        // pinned copy of d_series
+    long long* h_obs = nullptr;           // pinned copy of the observables (kObsBytes)
     int64_t series_cap = 0;               // pairs
     int sm_count = 148;
     int max_blocks = 148 * 8;           // grid cap: sm_count * blocks_per_sm
