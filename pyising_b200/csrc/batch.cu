@@ -175,18 +175,19 @@ __global__ void __launch_bounds__(256, ISING_BATCH_MIN_BLOCKS)
     batch_int8_kernel(const __grid_constant__ Int8LaunchN<N> P)
 {
     __shared__ u32 rt[kLookupWords];  // the lookup table of the decisions
-    // launched with programmatic stream serialization: wait for the previous kernel of the
-    // stream (every kernel of the engine's stream waits on its predecessor in turn, so this
-    // class's previous half-sweep has completed too), then let the next launch start
-    pdl_wait();
-    pdl_trigger();
+    // The lattice, its table and epoch come from the launch's parameters (whose first reads are
+    // slow) and a counter that changes between graph replays only: all before the wait.
     const Int8Desc& L = P.lat[find_lattice(P.lat, P.n)];
     if (threadIdx.x == 0) fill_lookup<NDIM, RULE>(rt, L.table);
-    __syncthreads();
     const long long epoch = P.epoch + (P.epoch_base ? *P.epoch_base : 0);
     bool meas;
     const Int8Half p = lattice_half(L, epoch, V, meas);
     const int b = (int)blockIdx.x;
+    __syncthreads();
+    // launched with programmatic stream serialization: wait for the class's previous half-sweep,
+    // then let the next launch start
+    pdl_wait();
+    pdl_trigger();
     const u32 s0 = (u32)(b - L.block_begin) * (u32)L.per_block;
     const u32 s1 = s0 + (u32)L.per_block < (u32)L.nslots ? s0 + (u32)L.per_block : (u32)L.nslots;
     long long m_acc = 0, e_acc = 0;
