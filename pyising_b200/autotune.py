@@ -12,8 +12,9 @@ by site, sweep and colour, and every schedule visits the same sites with the sam
                     bounded for 2, 3 or 4 resident blocks;
 * ``msc_waves``     msc: warps per resident warp (ranges or strip bands of the work-stack kernels);
 * ``graph_chunk``   sweeps per captured CUDA graph of an unmeasured run;
-* ``schedule``      ``"auto"`` (graphs), ``"launches"``, ``"persistent"`` or ``"temporal"``
-                    (2D int8: two sweeps per launch on shared-memory tiles).
+* ``schedule``      ``"auto"`` (tiles for small 2D lattices, else graphs), ``"launches"``,
+                    ``"persistent"`` or ``"temporal"`` (several half-sweeps per launch on
+                    shared-memory tiles).
 
 :func:`tune` measures them on a scratch lattice of the given shape (device seeded start, CUDA
 events on the simulation's stream) by coordinate descent from the defaults, and stores the best
