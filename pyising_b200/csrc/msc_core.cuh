@@ -531,15 +531,17 @@ __device__ __forceinline__ void level_pair_up(u32 re, u32 ro, const uint4& m, u3
 // local index, row parities those of the global rows, and rows -1 and `rows` of the opposite
 // colour are read from so.lo and so.hi instead of wrapping.
 // ODD: the parity of row y0 (+ colour), which every pair of rows starts with.
-template <int K, bool SLAB, bool ODD>
-__device__ __forceinline__ void msc_strip_pairs(const MscHalf& p, int strip, int y0, int y1,
+// ANY: rows of any number of words: each lane has its own column x and band [y0, y1) (of the same
+// even height and first parity), y1 = y0 for a lane without one; `pairs` is the most row pairs a
+// lane has.  A lane whose band is shorter repeats its last pair without storing it.
+template <int K, bool SLAB, bool ODD, bool ANY>
+__device__ __forceinline__ void msc_strip_pairs(const MscHalf& p, int x, int y0, int y1, int pairs,
                                                 StripSlots& q, const uint4* lvmask,
                                                 const SlabOffset& so)
 {
     const int lane = threadIdx.x & 31;
     const u32 lt_mask = (1u << lane) - 1u;
     const int nw = p.nw, rows = p.rows;
-    const int x = strip * 32 + lane;
     const int xr = x + 1 == nw ? 0 : x + 1, xl = x == 0 ? nw - 1 : x - 1;
     const u32 wg = SLAB ? (u32)so.w0 : 0u;
     // where the words of rows y and y + 1 are, from the current row pair
@@ -558,20 +560,26 @@ __device__ __forceinline__ void msc_strip_pairs(const MscHalf& p, int strip, int
         f_s0 = __ldg(oc + side0);
         f_s1 = __ldg(oc + (nw + side1));
     };
-    int y = y0;
+    int y = y0, left = pairs;
     fetch(y);
     u32 wa = (u32)((long long)y0 * nw + x);
     int n = 0;
     while (true) {
-        if (n < kPop && y < y1) {
+        if (n < kPop && left > 0) {
+            const bool act = !ANY || y < y1;
             const u64 o0 = f_o0, o1 = f_o1, d1 = f_d1, d2 = f_d2, s0 = f_s0, s1 = f_s1;
             const u64 hz0 = ODD ? ((c >> 1) | (s0 << 63)) : ((c << 1) | (s0 >> 63));
             const u64 hz1 = ODD ? ((d1 << 1) | (s1 >> 63)) : ((d1 >> 1) | (s1 << 63));
             u64* dst = own;
+            const u32 wi = wa;
+            --left;
+            if (!ANY || y + 2 < y1) {
+                own += 2 * (long long)nw;
+                oc += 2 * (long long)nw;
+                wa += 2u * (u32)nw;
+                if (left > 0) fetch(y + 2);
+            }
             y += 2;
-            own += 2 * (long long)nw;
-            oc += 2 * (long long)nw;
-            if (y < y1) fetch(y);
             const HalfSlices al = slice_half((u32)o0, (u32)c, (u32)hz0, (u32)up, (u32)d1);
             const HalfSlices ah = slice_half((u32)(o0 >> 32), (u32)(c >> 32), (u32)(hz0 >> 32),
                                              (u32)(up >> 32), (u32)(d1 >> 32));
@@ -580,14 +588,14 @@ __device__ __forceinline__ void msc_strip_pairs(const MscHalf& p, int strip, int
                                              (u32)(c >> 32), (u32)(d2 >> 32));
             up = d1;
             c = d2;
-            const u32 wb = wa + (u32)nw;
+            const u32 wb = wi + (u32)nw;
             u32 ual = ~0u, uah = ~0u, ubl = ~0u, ubh = ~0u;
             u32 aal = 0, aah = 0, abl = 0, abh = 0;
 #pragma unroll
             for (int b = K - 1; b >= 0; --b) {
                 const uint4 m = lvmask[b];
                 const u32x4 ra =
-                    philox4x32_10<true>(wg + wa, p.t, p.color, 1u + (u32)b, p.k0, p.k1);
+                    philox4x32_10<true>(wg + wi, p.t, p.color, 1u + (u32)b, p.k0, p.k1);
                 const u32x4 rb =
                     philox4x32_10<true>(wg + wb, p.t, p.color, 1u + (u32)b, p.k0, p.k1);
                 level_pair_up(ra.x, ra.z, m, al.a1, ual, aal);  // r0 | r1 << 32, r2 | r3 << 32
@@ -601,18 +609,20 @@ __device__ __forceinline__ void msc_strip_pairs(const MscHalf& p, int strip, int
             ubh &= ~bh.a2;
             const u32 ral = (u32)o0 ^ (al.a2 | aal), rah = (u32)(o0 >> 32) ^ (ah.a2 | aah);
             const u32 rbl = (u32)o1 ^ (bl.a2 | abl), rbh = (u32)(o1 >> 32) ^ (bh.a2 | abh);
-            const bool ka = (ual | uah) != 0, kb = (ubl | ubh) != 0;
+            const bool ka = act && (ual | uah) != 0, kb = act && (ubl | ubh) != 0;
             // every word is stored, decided or not: an undecided word's entry ends with the
             // store of its final value, and nothing else reads this colour during the
             // half-sweep (measured 0.6-0.8% faster than storing only the decided words here; in
             // the word-range walker 0.5% slower, so that one keeps the predicated store)
-            dst[0] = (u64)ral | ((u64)rah << 32);
-            dst[nw] = (u64)rbl | ((u64)rbh << 32);
+            if (act) {
+                dst[0] = (u64)ral | ((u64)rah << 32);
+                dst[nw] = (u64)rbl | ((u64)rbh << 32);
+            }
             const u32 kma = __ballot_sync(0xFFFFFFFFu, ka);
             const u32 kmb = __ballot_sync(0xFFFFFFFFu, kb);
             {
                 const int pos = ka ? n + __popc(kma & lt_mask) : kStripCap;
-                q.idx[pos] = wa;
+                q.idx[pos] = wi;
                 q.lp[pos] = (u32)K;
                 q.a1[pos] = (u64)al.a1 | ((u64)ah.a1 << 32);
                 q.und[pos] = (u64)ual | ((u64)uah << 32);
@@ -628,9 +638,8 @@ __device__ __forceinline__ void msc_strip_pairs(const MscHalf& p, int strip, int
                 q.res[pos] = (u64)rbl | ((u64)rbh << 32);
             }
             n += __popc(kmb);
-            wa += 2u * (u32)nw;
             __syncwarp();
-        } else if (y >= y1 && n <= 32) {
+        } else if (left == 0 && n <= 32) {
             if (n > 0) stack_drain(p, q, n, lvmask, wg);
             break;
         } else {
@@ -647,11 +656,12 @@ __device__ __forceinline__ void msc_strip_band(const MscHalf& p, int strip, int 
                                                const SlabOffset& so = {0, 0, nullptr, nullptr})
 {
     const int ye = y1 - ((y1 - y0) & 1);
+    const int x = strip * 32 + (int)(threadIdx.x & 31);
     if (ye > y0) {
         if ((y0 + (SLAB ? so.par0 : 0) + (int)p.color) & 1)
-            msc_strip_pairs<K, SLAB, true>(p, strip, y0, ye, q, lvmask, so);
+            msc_strip_pairs<K, SLAB, true, false>(p, x, y0, ye, (ye - y0) / 2, q, lvmask, so);
         else
-            msc_strip_pairs<K, SLAB, false>(p, strip, y0, ye, q, lvmask, so);
+            msc_strip_pairs<K, SLAB, false, false>(p, x, y0, ye, (ye - y0) / 2, q, lvmask, so);
     }
     if (ye < y1) {
         const long long w = (long long)ye * p.nw + strip * 32 + (int)(threadIdx.x & 31);

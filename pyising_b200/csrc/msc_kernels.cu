@@ -80,6 +80,50 @@ __global__ void __launch_bounds__(kQueueWarps * 32, MINB)
     }
 }
 
+// Rows of any number of words: lane g of the launch walks the rows of band g / nw in column g % nw,
+// so neighbouring lanes still read neighbouring words and no lane is without a column but at the
+// end.  Bands and rows are even, so every band starts with the same parity.
+//
+// Like the strips it is bound by the integer pipes; against the word ranges it has the levels of
+// two rows in flight per step, keeps the opposite colour's words of the next rows in registers
+// and needs no division or parity selection per word.  Measured on one B200, ranges -> lanes
+// (flips/ns): 4200x4224 1730 -> 2060, 6000x5248 1999 -> 2282, 6144^2 2384 -> 2822, 10000x9984
+// 2787 -> 3216, 20000x20096 3257 -> 4171, 160000x128 1621 -> 2288.  More and shorter bands (two
+// waves of warps) were slower from 5000x4992 on (20000x20096 3961).
+template <bool MEAS>
+__global__ void __launch_bounds__(kQueueWarps * 32, 2)
+    msc_lane_kernel(const MscHalf p_in, int band, int bands)
+{
+    MscHalf p = p_in;
+    __shared__ StripSlots q_all[kQueueWarps];
+    __shared__ uint4 lvmask[16];
+    if (threadIdx.x < 16) lvmask[threadIdx.x] = level_masks(p.thr4, p.thr8, threadIdx.x);
+    pdl_wait();  // the previous half-sweep has completed
+    pdl_trigger();
+    resolve_ctl(p);
+    __syncthreads();
+    const u32 g = blockIdx.x * (kQueueWarps * 32u) + threadIdx.x;
+    u32 b = g / (u32)p.nw;
+    int x = (int)(g - b * (u32)p.nw);
+    const bool valid = b < (u32)bands;
+    if (!valid) {
+        b = 0;
+        x = 0;
+    }
+    const int y0 = (int)b * band;
+    const int y1 = valid ? min(y0 + band, p.rows) : y0;
+    const SlabOffset none = {0, 0, nullptr, nullptr};
+    StripSlots& q = q_all[threadIdx.x >> 5];
+    if (p.color & 1) msc_strip_pairs<4, false, true, true>(p, x, y0, y1, band / 2, q, lvmask, none);
+    else msc_strip_pairs<4, false, false, true>(p, x, y0, y1, band / 2, q, lvmask, none);
+    if constexpr (MEAS) {
+        __syncwarp();  // the warp's words are final: measure them
+        long long m_acc = 0, e_acc = 0, calls = 0, wmax = 0;
+        for (int y = y0; y < y1; ++y) msc_word<false>(p, y, x, m_acc, e_acc, calls, wmax);
+        block_accumulate2(m_acc, e_acc, p.meas);
+    }
+}
+
 void msc_geometry(int rows, int nw, int max_blocks, dim3* grid, dim3* block)
 {
     int bx = 1;
@@ -160,13 +204,42 @@ static cudaError_t strip_launch(const MscHalf& p, int sm_count, int waves, cudaS
                   : launch_strip<false, K, MINB>(p, sm_count, waves, st);
 }
 
+// Words per SM from which rows that are not whole strips take the lane walk; a smaller half-sweep
+// is mostly latency, and the ranges put every word on a lane of its own.  Measured ranges / lanes
+// (flips/ns): 1152^2 (10,368 words) 234 / 208, 2000x1920 (30,000) 584 / 590, 3072^2 (73,728)
+// 1247 / 1417.
+constexpr long long kLaneWords = 256;
+
+template <bool MEAS>
+static cudaError_t launch_lanes(const MscHalf& p, int sm_count, int waves, cudaStream_t st)
+{
+    const long long words = (long long)p.rows * p.nw;
+    const long long lanes = (long long)(sm_count > 0 ? sm_count : 1) * 2 * kQueueWarps * 32 *
+                            (waves > 0 ? waves : 1);
+    long long band = (words + lanes - 1) / lanes;
+    band += band & 1;  // pairs of rows
+    if (band > p.rows) band = p.rows;
+    const long long bands = (p.rows + band - 1) / band;
+    const unsigned blocks =
+        (unsigned)((bands * p.nw + kQueueWarps * 32 - 1) / (kQueueWarps * 32));
+    return launch_pdl(msc_lane_kernel<MEAS>, dim3(blocks), dim3(kQueueWarps * 32), st, p, (int)band,
+                      (int)bands);
+}
+
 cudaError_t launch_msc_half(bool update, const MscHalf& p, int max_blocks, int sm_count,
                             int waves, cudaStream_t st, int kernel)
 {
     // the strip schedule needs rows of whole 32-word strips and word indices below 2^32
     const bool strip_ok = p.nw % 32 == 0 && (long long)p.rows * p.nw <= 0xFFFFFFFFll;
     // automatic: the strips (4 intake blocks, registers for 2 blocks per SM) wherever the rows
-    // hold whole 32-word strips, the word ranges elsewhere
+    // hold whole 32-word strips, elsewhere the lane walk, and the word ranges where that has too
+    // few words or their indices pass 2^32
+    const long long words = (long long)p.rows * p.nw;
+    const bool lanes_ok = p.nw % 32 != 0 && p.rows % 2 == 0 && words <= 0xFFFFFFFFll &&
+                          words >= kLaneWords * (sm_count > 0 ? sm_count : 1);
+    if (kernel == 0 && update && !p.stats && lanes_ok)
+        return p.meas ? launch_lanes<true>(p, sm_count, waves, st)
+                      : launch_lanes<false>(p, sm_count, waves, st);
     if (kernel == 0) kernel = strip_ok ? 2 : 1;
     if (update && !p.stats && strip_ok && kernel >= 2) {
         switch (kernel) {
