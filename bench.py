@@ -56,7 +56,7 @@ DESCRIPTION = {
                    "with (E, M) every 10 sweeps",
 }
 MEASURE_EVERY = {"int8_3d_256": 10}
-KERNEL = {"msc": "msc_strip_kernel", "int8": "int8_half_kernel"}
+KERNEL = {"msc": "msc_lane_kernel", "int8": "int8_half_kernel"}
 
 
 # ------------------------------------------------------------------------- helpers -------

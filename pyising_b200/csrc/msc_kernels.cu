@@ -89,7 +89,9 @@ __global__ void __launch_bounds__(kQueueWarps * 32, MINB)
 // and needs no division or parity selection per word.  Measured on one B200, ranges -> lanes
 // (flips/ns): 4200x4224 1730 -> 2060, 6000x5248 1999 -> 2282, 6144^2 2384 -> 2822, 10000x9984
 // 2787 -> 3216, 20000x20096 3257 -> 4171, 160000x128 1621 -> 2288.  More and shorter bands (two
-// waves of warps) were slower from 5000x4992 on (20000x20096 3961).
+// waves of warps) were slower from 5000x4992 on (20000x20096 3961).  Against the strips, which
+// walk rows of whole 32-word strips in the same steps: 4096^2 2115 both, 4600x12288 3083 -> 3155,
+// 8192^2 2971 -> 3038, 16384^2 4022 -> 4085.
 template <bool MEAS>
 __global__ void __launch_bounds__(kQueueWarps * 32, 2)
     msc_lane_kernel(const MscHalf p_in, int band, int bands)
@@ -204,7 +206,7 @@ static cudaError_t strip_launch(const MscHalf& p, int sm_count, int waves, cudaS
                   : launch_strip<false, K, MINB>(p, sm_count, waves, st);
 }
 
-// Words per SM from which rows that are not whole strips take the lane walk; a smaller half-sweep
+// Words per SM from which a half-sweep takes the lane walk; a smaller half-sweep
 // is mostly latency, and the ranges put every word on a lane of its own.  Measured ranges / lanes
 // (flips/ns): 1152^2 (10,368 words) 234 / 208, 2000x1920 (30,000) 584 / 590, 3072^2 (73,728)
 // 1247 / 1417.
@@ -231,11 +233,11 @@ cudaError_t launch_msc_half(bool update, const MscHalf& p, int max_blocks, int s
 {
     // the strip schedule needs rows of whole 32-word strips and word indices below 2^32
     const bool strip_ok = p.nw % 32 == 0 && (long long)p.rows * p.nw <= 0xFFFFFFFFll;
-    // automatic: the strips (4 intake blocks, registers for 2 blocks per SM) wherever the rows
-    // hold whole 32-word strips, elsewhere the lane walk, and the word ranges where that has too
-    // few words or their indices pass 2^32
+    // automatic: the lane walk; for few words the strips (4 intake blocks, registers for 2 blocks
+    // per SM) if the rows hold whole 32-word strips, else the word ranges; and these where the
+    // word indices pass 2^32
     const long long words = (long long)p.rows * p.nw;
-    const bool lanes_ok = p.nw % 32 != 0 && p.rows % 2 == 0 && words <= 0xFFFFFFFFll &&
+    const bool lanes_ok = p.rows % 2 == 0 && words <= 0xFFFFFFFFll &&
                           words >= kLaneWords * (sm_count > 0 ? sm_count : 1);
     if (kernel == 0 && update && !p.stats && lanes_ok)
         return p.meas ? launch_lanes<true>(p, sm_count, waves, st)

@@ -1,6 +1,6 @@
-"""The packed lane walk (rows that are not whole 32-word strips) against the oracle: one word per
-row, a few, more than a warp's; bands of two rows and of four with a shorter last one; the last
-warp partly without a column; and just below its range."""
+"""The packed lane walk against the oracle: one word per row, a few, a warp's, more; bands of two
+rows and of four with a shorter last one; the last warp partly without a column; and just below
+its range."""
 
 from __future__ import annotations
 
@@ -10,9 +10,10 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-# words per row: 1 (37886 rows: below the range), 3, 5, 33, 40; four-row bands with 3 and 65
+# words per row: 1 (37886 rows: below the range), 3, 5, 32, 33, 40; four-row bands with 3 and 65
 @pytest.mark.parametrize("shape", [(37886, 128), (37890, 128), (12634, 384), (7700, 640),
-                                   (1150, 4224), (970, 5120), (50522, 384), (2370, 8320)], ids=str)
+                                   (1186, 4096), (1150, 4224), (970, 5120), (50522, 384),
+                                   (2370, 8320)], ids=str)
 @pytest.mark.parametrize("beta", [0.1, 0.44068679350977147, 1.5])
 def test_msc_lanes(oracle_mod, shape, beta):
     from pyising_b200.backend import B200MultiSpin
