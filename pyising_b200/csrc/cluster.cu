@@ -533,6 +533,8 @@ static int cluster_setup(ising_sim* h)
 // T = 0: the single-level union-find in global memory (knob value 1).  Small tiles give many
 // CTAs and short trees, square-ish ones keep most bonds inside their tile.
 constexpr int kTileAuto = 512;
+constexpr int kTileMaxPositions = 6144;             // the knob's largest value
+constexpr int kTileSiteBytes = 2 * sizeof(int) + 1;  // shared memory per position
 
 static int cluster_tiles(const ising_sim* h, TileGeo* g)
 {
@@ -578,10 +580,11 @@ static int cluster_step(ising_sim* h, u32 t, u64 seed, u32 p_bond, bool flip)
     TileGeo g;
     const int tiles = cluster_tiles(h, &g);
     if (tiles > 0) {
-        const size_t smem = (size_t)g.R * g.W * (2 * sizeof(int) + 1);
-        if (smem > 48 * 1024) {
+        const size_t smem = (size_t)g.R * g.W * kTileSiteBytes;
+        if (smem > 48 * 1024) {  // one value for every thread and handle that shares the function
             const cudaError_t e = cudaFuncSetAttribute(
-                sw_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                sw_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                kTileMaxPositions * kTileSiteBytes);
             if (e != cudaSuccess) return cuda_fail(e, "cluster tile size");
         }
         // (many tiles: four warps each and more tiles per SM, 1024^2 61.6 / 65.5 us per update; few:

@@ -354,9 +354,12 @@ template <class Kernel, class... Args>
 static cudaError_t launch_tile(Kernel kernel, unsigned blocks, size_t smem, cudaStream_t st,
                                const Args&... args)
 {
-    if (smem > 32 * 1024) {  // above 48 KiB with the static arrays the limit must be raised
+    // Above 48 KiB with the static arrays the limit must be raised.  It belongs to the function,
+    // not to the launch: always the same value, so that no thread lowers it between another
+    // thread's call and its launch.
+    if (smem > 32 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(
-            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileMaxSmem);
         if (e != cudaSuccess) return e;
     }
     cudaLaunchConfig_t cfg = {};
