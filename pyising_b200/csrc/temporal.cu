@@ -470,7 +470,12 @@ static cudaError_t launch_tiles(const ising_sim* h, u32 t, int h0, int depth, in
 
 int temporal_scratch(ising_sim* h)
 {
-    for (int c = 0; c < 2; ++c) {
+    // Another stream may be under capture in a mode that forbids waiting for a stream: the
+    // allocation has nothing to do with it, so this thread does it in the relaxed mode.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    int rc = ISING_OK;
+    for (int c = 0; c < 2 && rc == ISING_OK; ++c) {
         if (h->tb_scratch[c]) continue;
         // on a stream that is then waited for: usable from any stream the handle is given later
         cudaError_t e =
@@ -479,10 +484,11 @@ int temporal_scratch(ising_sim* h)
         if (e != cudaSuccess) {
             cudaGetLastError();
             h->tb_scratch[c] = nullptr;
-            return fail(ISING_ERR_NOMEM, "allocation of the temporal schedule's second arrays");
+            rc = fail(ISING_ERR_NOMEM, "allocation of the temporal schedule's second arrays");
         }
     }
-    return ISING_OK;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return rc;
 }
 
 // `sweeps` sweeps from sweep t, (M, E) of the last one into meas (unless null): an even number of

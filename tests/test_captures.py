@@ -1,0 +1,42 @@
+"""Sweeps while CUDA graphs are captured: on another stream (a capture that has nothing to do with
+the lattice)."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+BETA_C_2D = 0.44068679350977147
+
+
+def pair(variant, shape):
+    from pyising_b200.backend import B200Int8, B200MultiSpin
+
+    cls = B200MultiSpin if variant == "msc" else B200Int8
+    return [cls(shape, BETA_C_2D, seed=3, init="philox") for _ in range(2)]
+
+
+def assert_same(a, b):
+    for x, y in zip(a.colour_arrays(), b.colour_arrays(), strict=True):
+        np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("variant,shape", [("msc", (64, 256)), ("int8", (62, 72)),
+                                           ("int8", (64, 64))], ids=str)
+def test_first_sweep_while_another_stream_is_captured(variant, shape):
+    import torch
+
+    a, b = pair(variant, shape)
+    a.synchronize()
+    x = torch.zeros(4, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):  # the global mode: no waiting for streams from this thread
+        x += 1
+        a.sweep(3)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [1.0] * 4
+    b.sweep(3)
+    assert_same(a, b)
