@@ -767,10 +767,17 @@ int ising_sweep(ising_sim* h, uint64_t t0, int64_t n_sweeps, int64_t measure_eve
         if (meas) ++k;
     }
     // Whole chunks of G sweeps replay one captured graph (G = the measurement interval, so each
-    // chunk ends with its measurement); the rest is launched directly.
+    // chunk ends with its measurement); the rest is launched directly.  Into a stream that the
+    // caller is capturing everything is launched directly: a capture cannot begin inside another.
     const int64_t G = measure_every > 0 ? measure_every : h->graph_chunk;
-    if (h->schedule != ISING_SCHEDULE_LAUNCHES && G <= kGraphChunkMax &&
-        n_sweeps - s0 >= 2 * G) {
+    bool graphs = h->schedule != ISING_SCHEDULE_LAUNCHES && G <= kGraphChunkMax &&
+                  n_sweeps - s0 >= 2 * G;
+    if (graphs) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        TRY_CUDA(cudaStreamIsCapturing(h->stream, &capture));
+        graphs = capture == cudaStreamCaptureStatusNone;
+    }
+    if (graphs) {
         cudaGraphExec_t exec = nullptr;
         int rc = chunk_graph(h, G, measure_every > 0, &exec);
         if (rc != ISING_OK) return rc;
