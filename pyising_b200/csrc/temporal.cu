@@ -29,6 +29,7 @@
 #include "capi_internal.h"
 #include "int8_core.cuh"
 #include "msc_core.cuh"
+#include "tile_plan.h"
 
 namespace ising {
 
@@ -499,17 +500,15 @@ cudaError_t launch_temporal_run(const ising_sim* h, u32 t, int64_t sweeps,
 {
     int band = 0, depth = 0;
     tile_shape(h, &band, &depth);
-    const int64_t halves = 2 * sweeps;
-    int64_t pairs = (halves + 2 * depth - 1) / (2 * depth);
+    const TileCuts cuts(2 * sweeps, depth);
     int64_t done = 0;
-    for (int64_t i = 0; i < 2 * pairs; ++i) {
-        const int64_t next = halves * (i + 1) / (2 * pairs);
-        const bool last = next == halves;
+    for (int64_t i = 0; i < cuts.launches; ++i) {
+        const int d = (int)cuts.depth(i);
         const cudaError_t e =
-            launch_tiles(h, t + (u32)(done >> 1), (int)(done & 1), (int)(next - done), band,
-                         last ? meas : nullptr, (i & 1) == 0);
+            launch_tiles(h, t + (u32)(done >> 1), (int)(done & 1), d, band,
+                         i + 1 == cuts.launches ? meas : nullptr, (i & 1) == 0);
         if (e != cudaSuccess) return e;
-        done = next;
+        done += d;
     }
     return cudaSuccess;
 }
