@@ -865,8 +865,11 @@ int ising_device_bytes(ising_sim* h, int64_t* bytes)
 {
     CHECK_HANDLE(h);
     if (!bytes) return fail(ISING_ERR_INVALID, "null output pointer");
-    *bytes = (int64_t)(2 * h->colour_bytes + 8 * sizeof(unsigned long long) +
-                       (size_t)h->series_cap * 2 * sizeof(long long));
+    size_t n = 2 * h->colour_bytes + 8 * sizeof(unsigned long long) +
+               (size_t)h->series_cap * 2 * sizeof(long long);
+    for (int c = 0; c < 2; ++c)
+        if (h->tb_scratch[c]) n += h->colour_bytes;  // the tiles' second pair
+    *bytes = (int64_t)n;
     return ISING_OK;
 }
 
