@@ -171,23 +171,24 @@ void clear_graphs(ising_sim* h)
     h->graphs.clear();
 }
 
-// Several half-sweeps per launch on shared-memory tiles: when asked for, and by default for
-// eligible lattices up to these many sites per colour (flips/ns, tiles / single half-sweeps).  A
-// launch knob of the single half-sweeps set by hand selects those (for int8 above kTemporalKnobs
-// sites).
-constexpr long long kTemporalInt8 = 6400 * 1024;  // 3500x3584 853 / 837, 4096^2 900 / 940
-constexpr long long kTemporalMsc = 4000 * 4096;   // 6000x5248 2202 / 1942, 6144^2 2309 / 2326
+// Several half-sweeps per launch on shared-memory tiles: when asked for, and by default where they
+// are the faster schedule (tiles_pay), up to these many sites per colour (flips/ns, tiles / single
+// half-sweeps): above them the single half-sweeps walk bands or lanes, which the rule's costs do not
+// describe.  A launch knob of the single half-sweeps set by hand selects those (for int8 above
+// kTemporalKnobs sites).
+constexpr long long kTemporalInt8 = 6400 * 1024;  // 3500x3584 866 / 839, 4096^2 917 / 940
+constexpr long long kTemporalMsc = 4000 * 4096;   // 5000x4992 2231 / 1876, 6144^2 2388 / 2815
 constexpr long long kTemporalKnobs = 512 * 1024;
 
 static bool use_temporal(const ising_sim* h)
 {
-    if (!temporal_ok(h)) return false;
-    if (h->schedule == ISING_SCHEDULE_TEMPORAL) return true;
+    if (h->schedule == ISING_SCHEDULE_TEMPORAL) return temporal_ok(h);
     if (h->schedule != ISING_SCHEDULE_AUTO) return false;
     const long long sites = h->rows * (long long)h->lh;
     if (h->variant == ISING_VARIANT_MSC)
-        return h->msc_kernel == 0 && h->msc_waves == 1 && sites <= kTemporalMsc;
-    return sites <= (h->band == 0 && h->vw == 16 ? kTemporalInt8 : kTemporalKnobs);
+        return h->msc_kernel == 0 && h->msc_waves == 1 && sites <= kTemporalMsc && temporal_pays(h);
+    return sites <= (h->band == 0 && h->vw == 16 ? kTemporalInt8 : kTemporalKnobs) &&
+           temporal_pays(h);
 }
 
 // The captured chunk of G sweeps of this handle: 2G half-sweeps with counters relative to the

@@ -3,6 +3,7 @@
 // thread kernel (the observables reduction and the call statistics).  Device code in
 // msc_core.cuh.
 #include "msc_core.cuh"
+#include "tile_plan.h"
 
 #ifndef ISING_MSC_MIN_BLOCKS
 #define ISING_MSC_MIN_BLOCKS 1
@@ -205,12 +206,6 @@ static cudaError_t strip_launch(const MscHalf& p, int sm_count, int waves, cudaS
     return p.meas ? launch_strip<true, K, MINB>(p, sm_count, waves, st)
                   : launch_strip<false, K, MINB>(p, sm_count, waves, st);
 }
-
-// Words per SM from which a half-sweep takes the lane walk; a smaller half-sweep
-// is mostly latency, and the ranges put every word on a lane of its own.  Measured ranges / lanes
-// (flips/ns): 1152^2 (10,368 words) 234 / 208, 2000x1920 (30,000) 584 / 590, 3072^2 (73,728)
-// 1247 / 1417.
-constexpr long long kLaneWords = 256;
 
 template <bool MEAS>
 static cudaError_t launch_lanes(const MscHalf& p, int sm_count, int waves, cudaStream_t st)

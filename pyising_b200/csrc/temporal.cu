@@ -23,7 +23,6 @@
 // rows are a few words.  Measured on one B200, flips/ns, single half-sweeps -> tiles: int8 256^2
 // 26 -> 48, 1024^2 303 -> 371, 2048^2 640 -> 680; msc 256^2 13 -> 41, 1152^2 236 -> 530, 2048^2
 // 728 -> 1212, 4096^2 1750 -> 2043.
-#include <cmath>
 #include <cstring>
 
 #include "capi_internal.h"
@@ -36,8 +35,6 @@ namespace ising {
 // One CTA of 16 warps per SM and 128 registers a thread: with two CTAs' worth of registers (64) the
 // pre-drawn random numbers spilled, and a step took up to 1.5 times as long.
 constexpr int kTileThreads = 512;
-constexpr int kTileMaxSmem = 200 * 1024;
-constexpr int kTileMaxDepth = 16;
 
 // Where a tile launch is: half-sweeps h0 .. h0 + depth - 1, counted from colour 0 of sweep p.t.
 struct TileRun {
@@ -319,36 +316,25 @@ static size_t tile_row_bytes(const ising_sim* h)
     return h->variant == ISING_VARIANT_MSC ? (size_t)h->nw * 8 : (size_t)h->pitch;
 }
 
-// The cost of a launch beside its steps, and of one row on one SM per 16 int8 sites and per 64-spin
-// word, as the depth rule needs them (they give the measured best depths: int8 256^2 8, 1024^2 4,
-// 2048^2 3; msc 512^2 8, 1152^2 5, 2048^2 4, 4096^2 3).
-constexpr double kLaunchUs = 1.0, kChunkUs = 2.0e-3, kWordUs = 4.1e-3;
-constexpr int kTileMinDepth = 3;
 // Tile words (of four int8 sites) up to which an int8 item is one word instead of four: 256^2
 // 44 / 38 flips/ns, 128^2 13 / 10; 1024^2 (above it) 287 / 355.
 constexpr int kTileWordItems = 1024;
 
-// Band and depth of this lattice's tiles; depth 0 if its rows do not fit.
-static void tile_shape(const ising_sim* h, int* band, int* depth)
+static TileRows tile_rows(const ising_sim* h)
 {
-    const int ly = h->ly, sms = h->sm_count > 0 ? h->sm_count : 1;
-    *band = (ly + sms - 1) / sms;
-    if (*band < 2) *band = 2;
-    const double row_us =
-        h->variant == ISING_VARIANT_MSC ? kWordUs * h->nw : kChunkUs * ((h->lh + 15) / 16);
-    int d = (int)(sqrt(kLaunchUs / row_us) + 0.5);
-    d = d < kTileMinDepth ? kTileMinDepth : (d > kTileMaxDepth ? kTileMaxDepth : d);
-    if (d > ly / 2) d = ly / 2;
-    while (d > 0 && 2 * (size_t)(*band + 2 * d) * tile_row_bytes(h) > (size_t)kTileMaxSmem) --d;
-    *depth = d;
+    const bool msc = h->variant == ISING_VARIANT_MSC;
+    return TileRows{msc, h->ly, msc ? h->nw : (h->lh + 15) / 16, tile_row_bytes(h),
+                    h->sm_count > 0 ? h->sm_count : 1};
 }
 
 bool temporal_ok(const ising_sim* h)
 {
-    if (h->ndim != 2) return false;
-    int band = 0, depth = 0;
-    tile_shape(h, &band, &depth);
-    return depth > 0;
+    return h->ndim == 2 && tile_shape(tile_rows(h)).depth > 0;
+}
+
+bool temporal_pays(const ising_sim* h)
+{
+    return h->ndim == 2 && tiles_pay(tile_rows(h));
 }
 
 template <class Kernel, class... Args>
@@ -498,14 +484,13 @@ int temporal_scratch(ising_sim* h)
 cudaError_t launch_temporal_run(const ising_sim* h, u32 t, int64_t sweeps,
                                 unsigned long long* meas)
 {
-    int band = 0, depth = 0;
-    tile_shape(h, &band, &depth);
-    const TileCuts cuts(2 * sweeps, depth);
+    const TileShape shape = tile_shape(tile_rows(h));
+    const TileCuts cuts(2 * sweeps, shape.depth);
     int64_t done = 0;
     for (int64_t i = 0; i < cuts.launches; ++i) {
         const int d = (int)cuts.depth(i);
         const cudaError_t e =
-            launch_tiles(h, t + (u32)(done >> 1), (int)(done & 1), d, band,
+            launch_tiles(h, t + (u32)(done >> 1), (int)(done & 1), d, shape.band,
                          i + 1 == cuts.launches ? meas : nullptr, (i & 1) == 0);
         if (e != cudaSuccess) return e;
         done += d;

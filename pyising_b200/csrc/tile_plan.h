@@ -1,9 +1,89 @@
-// How a run of sweeps is cut into tile launches: host arithmetic only, no CUDA.
+// Shape, cost and cutting of the temporal tiles: host arithmetic only, no CUDA.  Times are of one
+// half-sweep on one B200, in microseconds.
 #pragma once
 
+#include <cmath>
+#include <cstddef>
 #include <cstdint>
 
 namespace ising {
+
+constexpr int kTileMaxSmem = 200 * 1024;
+constexpr int kTileMaxDepth = 16;
+constexpr int kTileMinDepth = 3;
+
+// A 2D lattice as the plan sees it: rows of `units` 16-site chunks (int8) or 64-spin words (msc).
+struct TileRows {
+    bool msc;
+    int ly, units;
+    size_t row_bytes;  // of one colour
+    int sms;
+};
+
+// Rows that a CTA writes back and half-sweeps per launch; depth 0: the rows do not fit.
+struct TileShape {
+    int band, depth;
+};
+
+// The depth rule: the cost of a launch beside its steps, and of one row on one SM per chunk and
+// word, with which it gives the measured best depths (int8 256^2 8, 1024^2 4, 2048^2 3; msc 512^2
+// 8, 1152^2 5, 2048^2 4, 4096^2 3).
+constexpr double kLaunchUs = 1.0, kDepthChunkUs = 2.0e-3, kDepthWordUs = 4.1e-3;
+
+inline TileShape tile_shape(const TileRows& r)
+{
+    TileShape s;
+    s.band = (r.ly + r.sms - 1) / r.sms;
+    if (s.band < 2) s.band = 2;
+    const double row_us = (r.msc ? kDepthWordUs : kDepthChunkUs) * r.units;
+    int d = (int)(std::sqrt(kLaunchUs / row_us) + 0.5);
+    d = d < kTileMinDepth ? kTileMinDepth : (d > kTileMaxDepth ? kTileMaxDepth : d);
+    if (d > r.ly / 2) d = r.ly / 2;
+    while (d > 0 && 2 * (size_t)(s.band + 2 * d) * r.row_bytes > (size_t)kTileMaxSmem) --d;
+    s.depth = d;
+    return s;
+}
+
+// A step on tiles: a chain of latencies, its share of the launch, and the rows that a CTA updates
+// (band + depth - 1 on average).  A lattice of few rows has few CTAs, each of which recomputes
+// nearly as many rows as it keeps.
+constexpr double kTileChunkUs = 2.2e-3, kTileWordUs = 3.4e-3;
+
+inline double tile_half_us(const TileRows& r, const TileShape& s)
+{
+    const double row_us = (r.msc ? kTileWordUs : kTileChunkUs) * r.units;
+    return (r.msc ? 0.5 : 0.4) + kLaunchUs / s.depth + row_us * (s.band + s.depth - 1);
+}
+
+// Words per SM from which a single half-sweep takes the lane walk; a smaller one is mostly latency,
+// and the ranges put every word on a lane of its own.  Measured ranges / lanes (flips/ns): 1152^2
+// (10,368 words) 234 / 208, 2000x1920 (30,000) 584 / 590, 3072^2 (73,728) 1267 / 1438.
+constexpr int kLaneWords = 256;
+
+// A half-sweep of its own, spread over all SMs.  int8: one chunk per thread.  msc: word ranges or
+// strips up to kLaneWords words per SM, then the lane walk, whose lanes (two blocks of 256 per SM)
+// take an even number of rows each.
+inline double single_half_us(const TileRows& r)
+{
+    const double units = (double)r.ly * r.units;
+    if (!r.msc) return 1.45 + kTileChunkUs * units / r.sms;
+    const double fill = units / ((double)kLaneWords * r.sms);
+    if (fill < 1) return 2.45 + 0.4 * fill + (r.units % 32 == 0 ? 0.6 : 0.0);
+    const double rows = 2 * std::ceil(units / (512.0 * r.sms) / 2);
+    return (units / rows / 256 > r.sms ? 2.35 : 1.15) + 1.07 * rows;
+}
+
+// Whether tiles beat single half-sweeps.  Measured, flips/ns, tiles / single half-sweeps (and the
+// two times of the model): int8 1024^2 391 / 300 (1.35, 1.94), 64x1024 34 / 26 (1.00, 1.48), 512x4096
+// 451 / 431 (2.42, 2.42), 64x4096 77 / 91 (1.86, 1.57), 64x16384 102 / 265 (5.24, 1.94), 1024x8192
+// 713 / 789 (5.80, 5.35); msc 1152^2 571 / 239 (1.07, 2.56), 4096^2 2116 / 1861 (4.10, 4.49), 6000x5248
+// 2282 / 2364 (6.83, 6.63), 64x8192 169 / 84 (1.70, 3.09), 64x65536 285 / 622 (7.80, 3.40), 128x32768
+// 523 / 622 (4.31, 3.40).
+inline bool tiles_pay(const TileRows& r)
+{
+    const TileShape s = tile_shape(r);
+    return s.depth > 0 && tile_half_us(r, s) <= single_half_us(r);
+}
 
 // A run of `halves` half-sweeps in an even number of launches of about the same depth, at most
 // `depth` each.

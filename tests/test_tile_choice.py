@@ -32,3 +32,17 @@ def second_pair(variant, shape, schedule="auto"):
 def test_device_bytes_count_the_second_pair(variant, shape):
     assert second_pair(variant, shape, "temporal")
     assert not second_pair(variant, shape, "launches")
+
+
+# wide, low lattices: few bands of rows for the SMs, and most of a band's work is its halo
+@pytest.mark.parametrize("variant,shape,tiles", [
+    ("int8", (1024, 1024), True), ("int8", (1500, 2488), True), ("msc", (1152, 1152), True),
+    ("msc", (4096, 4096), True), ("int8", (64, 16384), False), ("int8", (256, 8192), False),
+    ("msc", (64, 65536), False), ("msc", (128, 32768), False), ("msc", (6000, 5248), False),
+], ids=str)
+def test_automatic_schedule_takes_tiles_where_they_are_faster(variant, shape, tiles):
+    import torch
+
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the choice depends on the number of SMs")
+    assert second_pair(variant, shape) == tiles

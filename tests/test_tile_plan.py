@@ -22,6 +22,16 @@ extern "C" void cuts(long long halves, int depth, long long* out)
     out[3] = c.launches ? c.depth(0) : 0;
     out[4] = c.launches ? c.depth(c.launches - 1) : 0;
 }
+extern "C" int plan(int msc, int ly, int units, int row_bytes, int sms, int* shape, double* us)
+{
+    const ising::TileRows r{msc != 0, ly, units, (size_t)row_bytes, sms};
+    const ising::TileShape s = ising::tile_shape(r);
+    shape[0] = s.band;
+    shape[1] = s.depth;
+    us[0] = s.depth > 0 ? ising::tile_half_us(r, s) : 0.0;
+    us[1] = ising::single_half_us(r);
+    return ising::tiles_pay(r);
+}
 """
 
 
@@ -48,3 +58,38 @@ def test_cuts_cover_the_run(plan, sweeps, depth):
     if sweeps:
         assert 1 <= last <= first <= depth
         assert launches - 2 < 2 * sweeps / depth  # no more launches than the depth asks for
+
+
+def choose(lib, variant, shape, sms=148):
+    ly, lx = shape
+    units = lx // 128 if variant == "msc" else -(-lx // 32)
+    row_bytes = units * (8 if variant == "msc" else 16)
+    out, us = (ctypes.c_int * 2)(), (ctypes.c_double * 2)()
+    pays = lib.plan(int(variant == "msc"), ly, units, row_bytes, sms, out, us)
+    band, depth = out
+    assert band * sms >= ly and band >= 2
+    assert 0 <= depth <= 16 and 2 * depth <= ly
+    assert 2 * (band + 2 * depth) * row_bytes <= 200 * 1024 or depth == 0
+    return bool(pays), tuple(us)
+
+
+# the faster schedule as measured on a B200 (by more than a few percent), wide and low lattices
+# among them: these have few bands, and a band's halo rows are recomputed
+@pytest.mark.parametrize("variant,shape,tiles", [
+    ("int8", (64, 64), True), ("int8", (1024, 1024), True), ("int8", (1500, 2488), True),
+    ("int8", (3000, 3000), True), ("int8", (3500, 3584), True), ("int8", (64, 1024), True),
+    ("int8", (128, 2048), True), ("int8", (512, 4096), True), ("int8", (65536, 64), True),
+    ("int8", (8192, 1024), True), ("int8", (2, 32768), False), ("int8", (16, 4096), False),
+    ("int8", (16, 32768), False), ("int8", (64, 4096), False), ("int8", (64, 16384), False),
+    ("int8", (128, 16384), False), ("int8", (256, 8192), False), ("int8", (256, 32768), False),
+    ("int8", (512, 8192), False), ("int8", (1024, 8192), False), ("int8", (2, 10**6), False),
+    ("msc", (128, 128), True), ("msc", (1152, 1152), True), ("msc", (2048, 2048), True),
+    ("msc", (3072, 3072), True), ("msc", (4096, 4096), True), ("msc", (4600, 4608), True),
+    ("msc", (5000, 4992), True), ("msc", (16, 16384), True), ("msc", (64, 8192), True),
+    ("msc", (128, 4096), True), ("msc", (2048, 8192), True), ("msc", (65536, 128), True),
+    ("msc", (6000, 5248), False), ("msc", (2, 131072), False), ("msc", (16, 131072), False),
+    ("msc", (64, 65536), False), ("msc", (128, 32768), False), ("msc", (256, 32768), False),
+], ids=str)
+def test_tiles_where_they_are_faster(plan, variant, shape, tiles):
+    pays, us = choose(plan, variant, shape)
+    assert pays == tiles, us
