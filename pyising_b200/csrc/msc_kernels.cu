@@ -2,8 +2,8 @@
 // measured half-sweep measures each warp's words after updating them) and the one-word-per-
 // thread kernel (the observables reduction and the call statistics).  Device code in
 // msc_core.cuh.
+#include "lane_plan.h"
 #include "msc_core.cuh"
-#include "tile_plan.h"
 
 #ifndef ISING_MSC_MIN_BLOCKS
 #define ISING_MSC_MIN_BLOCKS 1
@@ -207,15 +207,15 @@ static cudaError_t strip_launch(const MscHalf& p, int sm_count, int waves, cudaS
                   : launch_strip<false, K, MINB>(p, sm_count, waves, st);
 }
 
-template <bool MEAS>
-static cudaError_t launch_lanes(const MscHalf& p, int sm_count, int waves, cudaStream_t st)
+// Lanes resident at a time (two blocks per SM), times the waves asked for.
+static long long resident_lanes(int sms, int waves)
 {
-    const long long words = (long long)p.rows * p.nw;
-    const long long lanes = (long long)(sm_count > 0 ? sm_count : 1) * 2 * kQueueWarps * 32 *
-                            (waves > 0 ? waves : 1);
-    long long band = (words + lanes - 1) / lanes;
-    band += band & 1;  // pairs of rows
-    if (band > p.rows) band = p.rows;
+    return (long long)sms * 2 * kQueueWarps * 32 * (waves > 0 ? waves : 1);
+}
+
+template <bool MEAS>
+static cudaError_t launch_lanes(const MscHalf& p, long long band, cudaStream_t st)
+{
     const long long bands = (p.rows + band - 1) / band;
     const unsigned blocks =
         (unsigned)((bands * p.nw + kQueueWarps * 32 - 1) / (kQueueWarps * 32));
@@ -230,13 +230,15 @@ cudaError_t launch_msc_half(bool update, const MscHalf& p, int max_blocks, int s
     const bool strip_ok = p.nw % 32 == 0 && (long long)p.rows * p.nw <= 0xFFFFFFFFll;
     // automatic: the lane walk; for few words the strips (4 intake blocks, registers for 2 blocks
     // per SM) if the rows hold whole 32-word strips, else the word ranges; and these where the
-    // word indices pass 2^32
-    const long long words = (long long)p.rows * p.nw;
-    const bool lanes_ok = p.rows % 2 == 0 && words <= 0xFFFFFFFFll &&
-                          words >= kLaneWords * (sm_count > 0 ? sm_count : 1);
-    if (kernel == 0 && update && !p.stats && lanes_ok)
-        return p.meas ? launch_lanes<true>(p, sm_count, waves, st)
-                      : launch_lanes<false>(p, sm_count, waves, st);
+    // word indices pass 2^32 or the walk's bands would leave many lanes idle
+    if (kernel == 0 && update && !p.stats) {
+        const int sms = sm_count > 0 ? sm_count : 1;
+        const long long band = lane_band(p.rows, p.nw, resident_lanes(sms, waves), sms);
+        if (band > 0)
+            return p.meas ? launch_lanes<true>(p, band, st) : launch_lanes<false>(p, band, st);
+        const bool few = (long long)p.rows * p.nw < (long long)kLaneWords * sms;
+        kernel = strip_ok && few ? 2 : 1;
+    }
     if (kernel == 0) kernel = strip_ok ? 2 : 1;
     if (update && !p.stats && strip_ok && kernel >= 2) {
         switch (kernel) {

@@ -6,6 +6,8 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "lane_plan.h"
+
 namespace ising {
 
 constexpr int kTileMaxSmem = 200 * 1024;
@@ -54,11 +56,6 @@ inline double tile_half_us(const TileRows& r, const TileShape& s)
     const double row_us = (r.msc ? kTileWordUs : kTileChunkUs) * r.units;
     return (r.msc ? 0.5 : 0.4) + kLaunchUs / s.depth + row_us * (s.band + s.depth - 1);
 }
-
-// Words per SM from which a single half-sweep takes the lane walk; a smaller one is mostly latency,
-// and the ranges put every word on a lane of its own.  Measured ranges / lanes (flips/ns): 1152^2
-// (10,368 words) 234 / 208, 2000x1920 (30,000) 584 / 590, 3072^2 (73,728) 1267 / 1438.
-constexpr int kLaneWords = 256;
 
 // A half-sweep of its own, spread over all SMs.  int8: one chunk per thread.  msc: word ranges or
 // strips up to kLaneWords words per SM, then the lane walk, whose lanes (two blocks of 256 per SM)

@@ -1,4 +1,5 @@
-"""The host arithmetic of the temporal tiles (csrc/tile_plan.h), compiled for the CPU."""
+"""The host arithmetic of the temporal tiles (csrc/tile_plan.h) and of the packed lane walk
+(csrc/lane_plan.h), compiled for the CPU."""
 
 from __future__ import annotations
 
@@ -21,6 +22,10 @@ extern "C" void cuts(long long halves, int depth, long long* out)
     out[2] = c.longer;
     out[3] = c.launches ? c.depth(0) : 0;
     out[4] = c.launches ? c.depth(c.launches - 1) : 0;
+}
+extern "C" long long lane_band(long long rows, long long nw, long long lanes, long long sms)
+{
+    return ising::lane_band(rows, nw, lanes, sms);
 }
 extern "C" int plan(int msc, int ly, int units, int row_bytes, int sms, int* shape, double* us)
 {
@@ -93,3 +98,37 @@ def choose(lib, variant, shape, sms=148):
 def test_tiles_where_they_are_faster(plan, variant, shape, tiles):
     pays, us = choose(plan, variant, shape)
     assert pays == tiles, us
+
+
+LANES = 148 * 512
+
+
+@pytest.mark.parametrize("nw", [1, 2, 3, 5, 31, 32, 49, 128, 1000, 40000, 80000])
+@pytest.mark.parametrize("fill", [0.3, 0.51, 1.0, 1.9, 2.03, 3.0, 3.3, 3.99, 4.05, 5.9, 8.1, 14.2,
+                                  19.99, 20.0, 40.0, 100.0])
+def test_lane_bands_fit_the_resident_lanes(plan, nw, fill):
+    plan.lane_band.restype = ctypes.c_longlong
+    rows = max(2, int(fill * LANES / nw) // 2 * 2)
+    args = [ctypes.c_longlong(x) for x in (rows, nw, LANES, 148)]
+    band = plan.lane_band(*args)
+    words = rows * nw
+    if words < 256 * 148:
+        assert band == 0
+        return
+    assert band % 2 == 0 and 0 <= band <= rows
+    if nw <= 128 and not 2 < words / LANES < 3.3:
+        assert band > 0  # word ranges only where the walk would leave many lanes idle
+    if band > 2:
+        assert -(-rows // band) * nw <= LANES  # one wave: no block left over
+        assert nw > 1 or band % 16
+        assert words >= 0.4 * LANES * band  # and not mostly idle
+
+
+@pytest.mark.parametrize("shape,band", [((505172, 384), 22), ((2402, 8192), 0), ((3552, 8192), 0),
+                                        ((4616, 8192), 4), ((4794, 8192), 6), ((650, 8192), 2),
+                                        ((4600, 4608), 0), ((6000, 5248), 4), ((16384, 16384), 28),
+                                        ((1152, 1152), 0)], ids=str)
+def test_lane_bands(plan, shape, band):
+    plan.lane_band.restype = ctypes.c_longlong
+    args = [ctypes.c_longlong(x) for x in (shape[0], shape[1] // 128, LANES, 148)]
+    assert plan.lane_band(*args) == band
