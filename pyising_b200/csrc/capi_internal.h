@@ -93,8 +93,8 @@ int int8_default_band(long long rows, int ly, int cpr, int sm_count);
 unsigned int8_band_geometry(Int8Half& p, int max_blocks, int sm_count);
 cudaError_t launch_int8_half(int ndim, int rule, const Int8Half& p, int max_blocks, int sm_count,
                              cudaStream_t st);
-// kernel: 0 = automatic (the strip schedule where the rows hold whole 32-word strips), 1 = the
-// range schedule, 2..7 = the strip schedule with (Philox blocks per word at intake, resident
+// kernel: 0 = automatic (the lane walk, or the range schedule: lane_plan.h), 1 = the range
+// schedule, 2..7 = the strip schedule with (Philox blocks per word at intake, resident
 // blocks the registers are bounded for) = (4, 2), (4, 3), (4, 4), (3, 2), (3, 3), (3, 4).
 cudaError_t launch_msc_half(bool update, const MscHalf& p, int max_blocks, int sm_count,
                             int waves, cudaStream_t st, int kernel = 0);

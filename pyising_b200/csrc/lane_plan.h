@@ -5,7 +5,8 @@ namespace ising {
 
 // Words per SM from which a half-sweep takes the lane walk; a smaller one is mostly latency, and
 // the ranges put every word on a lane of its own.  Measured ranges / lanes (flips/ns): 1152^2
-// (10,368 words) 234 / 208, 2000x1920 (30,000) 584 / 590, 3072^2 (73,728) 1267 / 1438.
+// (10,368 words) 234 / 208, 2000x1920 (30,000) 584 / 590, 3072^2 (73,728) 1267 / 1438.  (Strips, for
+// rows of whole 32-word strips, are slower still on few words: 64x8192 99 / 83, 64x65536 724 / 618.)
 constexpr int kLaneWords = 256;
 
 // Rows per lane of the lane walk (an even number) on `lanes` resident lanes; 0: word ranges.

@@ -228,18 +228,15 @@ cudaError_t launch_msc_half(bool update, const MscHalf& p, int max_blocks, int s
 {
     // the strip schedule needs rows of whole 32-word strips and word indices below 2^32
     const bool strip_ok = p.nw % 32 == 0 && (long long)p.rows * p.nw <= 0xFFFFFFFFll;
-    // automatic: the lane walk; for few words the strips (4 intake blocks, registers for 2 blocks
-    // per SM) if the rows hold whole 32-word strips, else the word ranges; and these where the
-    // word indices pass 2^32 or the walk's bands would leave many lanes idle
+    // automatic: the lane walk; the word ranges for few words, where the word indices pass 2^32 and
+    // where the walk's bands would leave many lanes idle
     if (kernel == 0 && update && !p.stats) {
         const int sms = sm_count > 0 ? sm_count : 1;
         const long long band = lane_band(p.rows, p.nw, resident_lanes(sms, waves), sms);
         if (band > 0)
             return p.meas ? launch_lanes<true>(p, band, st) : launch_lanes<false>(p, band, st);
-        const bool few = (long long)p.rows * p.nw < (long long)kLaneWords * sms;
-        kernel = strip_ok && few ? 2 : 1;
+        kernel = 1;
     }
-    if (kernel == 0) kernel = strip_ok ? 2 : 1;
     if (update && !p.stats && strip_ok && kernel >= 2) {
         switch (kernel) {
         case 2: return strip_launch<4, 2>(p, sm_count, waves, st);

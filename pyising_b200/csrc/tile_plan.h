@@ -49,7 +49,7 @@ inline TileShape tile_shape(const TileRows& r)
 // A step on tiles: a chain of latencies, its share of the launch, and the rows that a CTA updates
 // (band + depth - 1 on average).  A lattice of few rows has few CTAs, each of which recomputes
 // nearly as many rows as it keeps.
-constexpr double kTileChunkUs = 2.2e-3, kTileWordUs = 3.4e-3;
+constexpr double kTileChunkUs = 2.2e-3, kTileWordUs = 3.35e-3;
 
 inline double tile_half_us(const TileRows& r, const TileShape& s)
 {
@@ -57,15 +57,15 @@ inline double tile_half_us(const TileRows& r, const TileShape& s)
     return (r.msc ? 0.5 : 0.4) + kLaunchUs / s.depth + row_us * (s.band + s.depth - 1);
 }
 
-// A half-sweep of its own, spread over all SMs.  int8: one chunk per thread.  msc: word ranges or
-// strips up to kLaneWords words per SM, then the lane walk, whose lanes (two blocks of 256 per SM)
-// take an even number of rows each.
+// A half-sweep of its own, spread over all SMs.  int8: one chunk per thread.  msc: word ranges up to
+// kLaneWords words per SM, then the lane walk, whose lanes (two blocks of 256 per SM) take an even
+// number of rows each.
 inline double single_half_us(const TileRows& r)
 {
     const double units = (double)r.ly * r.units;
     if (!r.msc) return 1.45 + kTileChunkUs * units / r.sms;
     const double fill = units / ((double)kLaneWords * r.sms);
-    if (fill < 1) return 2.45 + 0.4 * fill + (r.units % 32 == 0 ? 0.6 : 0.0);
+    if (fill < 1) return 2.55 + 0.4 * fill;
     const double rows = 2 * std::ceil(units / (512.0 * r.sms) / 2);
     return (units / rows / 256 > r.sms ? 2.35 : 1.15) + 1.07 * rows;
 }
@@ -73,9 +73,9 @@ inline double single_half_us(const TileRows& r)
 // Whether tiles beat single half-sweeps.  Measured, flips/ns, tiles / single half-sweeps (and the
 // two times of the model): int8 1024^2 391 / 300 (1.35, 1.94), 64x1024 34 / 26 (1.00, 1.48), 512x4096
 // 451 / 431 (2.42, 2.42), 64x4096 77 / 91 (1.86, 1.57), 64x16384 102 / 265 (5.24, 1.94), 1024x8192
-// 713 / 789 (5.80, 5.35); msc 1152^2 571 / 239 (1.07, 2.56), 4096^2 2116 / 1861 (4.10, 4.49), 6000x5248
-// 2282 / 2364 (6.83, 6.63), 64x8192 169 / 84 (1.70, 3.09), 64x65536 285 / 622 (7.80, 3.40), 128x32768
-// 523 / 622 (4.31, 3.40).
+// 713 / 789 (5.80, 5.35); msc 1152^2 571 / 239 (1.06, 2.66), 4096^2 2116 / 1861 (4.05, 4.49), 6000x5248
+// 2282 / 2364 (6.74, 6.63), 64x8192 169 / 99 (1.69, 2.59), 64x65536 285 / 724 (7.69, 2.90), 128x32768
+// 523 / 731 (4.26, 2.90).
 inline bool tiles_pay(const TileRows& r)
 {
     const TileShape s = tile_shape(r);
