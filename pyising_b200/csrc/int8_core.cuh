@@ -374,7 +374,9 @@ __device__ __forceinline__ void int8_band_row(const Int8Half& p, const BandRow& 
 // opposite-colour rows a row needs (y-1, y, y+1) slide down the band, so each row loads and masks
 // one new opposite-colour row (plus the planes z +- 1 in 3D) instead of three.  A band of an even
 // number of rows takes two rows per step: the row parity, which side the horizontal neighbours
-// are on, is then fixed in the code, and the sliding rows are renamed every second row only.
+// are on, is then fixed in the code, and the sliding rows are renamed every second row only.  Not
+// so padded rows that are measured: two such rows in flight need more than the 64 registers of four
+// blocks per SM (spilled, a measured sweep of 3D 300x300x304 took 58.4 us, row by row 44.7).
 template <int V, int NDIM, int RULE, bool MIXED, bool MEAS>
 __device__ __forceinline__ void int8_band(const Int8Half& p, int z, int y0, int y1, int j0,
                                           const u32* rt, long long& m_acc, long long& e_acc)
@@ -423,10 +425,12 @@ __device__ __forceinline__ void int8_band(const Int8Half& p, int z, int y0, int 
             c = d2;
         }
     };
-    if (((y0 | y1) & 1) == 0) {
-        if (par0) pairs(std::integral_constant<int, 1>{});
-        else pairs(std::integral_constant<int, 0>{});
-        return;
+    if constexpr (!(MIXED && MEAS)) {
+        if (((y0 | y1) & 1) == 0) {
+            if (par0) pairs(std::integral_constant<int, 1>{});
+            else pairs(std::integral_constant<int, 0>{});
+            return;
+        }
     }
 #pragma unroll 1
     for (int y = y0; y < y1; ++y) {
