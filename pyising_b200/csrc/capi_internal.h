@@ -89,7 +89,6 @@ int selftest_bounded_wait(int device, int* timed_out);
 
 // kernel launchers
 int int8_chunk_width(int lh);
-int int8_default_band(long long rows, int ly, int cpr, int sm_count);
 unsigned int8_band_geometry(Int8Half& p, int max_blocks, int sm_count);
 cudaError_t launch_int8_half(int ndim, int rule, const Int8Half& p, int max_blocks, int sm_count,
                              cudaStream_t st);

@@ -16,6 +16,7 @@
 // 2D 16384^2 1030 -> 1211, 3D 512^3 heat bath 818 -> 1062, 3D 256^3 heat bath 710 -> 858.
 //
 // Lattices below kOneChunkRows chunks run one chunk per thread instead (int8_one_kernel).
+#include "band_plan.h"
 #include "int8_core.cuh"
 
 namespace ising {
@@ -135,16 +136,6 @@ static cudaError_t launch_v(int ndim, int rule, const Int8Plan& plan, const Int8
 
 // Chunk width used for a row of lh bytes: the widest of 16/8/4 that divides it.
 int int8_chunk_width(int lh) { return lh % 16 == 0 ? 16 : (lh % 8 == 0 ? 8 : 4); }
-
-// Default band height: the longest of 16, 8, 4, 2, 1 rows whose slots still give every SM one
-// wave of resident threads (4 blocks of 256 at 64 registers).
-int int8_default_band(long long rows, int ly, int cpr, int sm_count)
-{
-    const long long want = 1024LL * sm_count;
-    int b = 16;
-    while (b > 1 && (rows / ly) * ((ly + b - 1) / b) * (long long)cpr < want) b >>= 1;
-    return b;
-}
 
 // Fills in the band fields of p (band from p.band, or the default when p.band <= 0) and
 // returns the grid: one block per 256 slots, at most max_blocks.

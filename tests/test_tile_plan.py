@@ -1,5 +1,5 @@
 """The host arithmetic of the temporal tiles (csrc/tile_plan.h) and of the packed lane walk
-(csrc/lane_plan.h), compiled for the CPU."""
+(csrc/lane_plan.h), and the bands of int8 half-sweeps (csrc/band_plan.h), compiled for the CPU."""
 
 from __future__ import annotations
 
@@ -13,6 +13,7 @@ import pytest
 CSRC = Path(__file__).resolve().parents[1] / "pyising_b200" / "csrc"
 
 SHIM = r"""
+#include "band_plan.h"
 #include "tile_plan.h"
 extern "C" void cuts(long long halves, int depth, long long* out)
 {
@@ -26,6 +27,10 @@ extern "C" void cuts(long long halves, int depth, long long* out)
 extern "C" long long lane_band(long long rows, long long nw, long long lanes, long long sms)
 {
     return ising::lane_band(rows, nw, lanes, sms);
+}
+extern "C" int band(long long rows, int ly, int cpr, int sms)
+{
+    return ising::int8_default_band(rows, ly, cpr, sms);
 }
 extern "C" int plan(int msc, int ly, int units, int row_bytes, int sms, int* shape, double* us)
 {
@@ -132,3 +137,19 @@ def test_lane_bands(plan, shape, band):
     plan.lane_band.restype = ctypes.c_longlong
     args = [ctypes.c_longlong(x) for x in (shape[0], shape[1] // 128, LANES, 148)]
     assert plan.lane_band(*args) == band
+
+
+# the measured best heights (or, in brackets, those within a few percent of it)
+@pytest.mark.parametrize("shape,best", [
+    ((16384, 16384), [16]), ((12000, 12000), [8, 16]), ((9000, 9000), [4, 8]),
+    ((8192, 8192), [4, 8]), ((7000, 7000), [4]), ((5000, 5000), [2]), ((4096, 4096), [2]),
+    ((2000000, 32), [4]), ((256, 256, 256), [2]), ((300, 300, 304), [2]), ((400, 400, 416), [4]),
+    ((448, 448, 448), [4]), ((512, 512, 512), [8, 16]), ((640, 640, 640), [16]),
+    ((1000, 1000, 24), [2]), ((2000, 2000, 32), [2]), ((100, 1000, 1000), [4]), ((64, 64), [1]),
+], ids=str)
+def test_default_band(plan, shape, best):
+    rows = 1
+    for extent in shape[:-1]:
+        rows *= extent
+    got = plan.band(ctypes.c_longlong(rows), shape[-2], -(-shape[-1] // 32), 148)
+    assert got in best
