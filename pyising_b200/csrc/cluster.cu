@@ -30,17 +30,19 @@
 // Labels are int32 (lattices of fewer than 2^31 sites).  Every retry loop is bounded: a thread
 // that exceeds the bound sets the error word and stops, and the host reports ISING_ERR_TIMEOUT.
 #include "capi_internal.h"
+#include "tile_forest.h"
 
 namespace ising {
 
 constexpr u32 kBondTag = 0x53570001u;  // Philox counter word 2 of the bond uniforms
 constexpr u32 kFlipTag = 0x53570002u;  // ... of the cluster flip bits
 // Bounded loops: one union (its finds and retries) or one root walk may take at most kStepLimit
-// steps (about 0.3 s of dependent L2 reads; legitimate walks are far shorter), and every loop
-// gives up as soon as any thread has set the error word, which it reads every kErrPoll steps.
-// A thread that runs out sets the error word, so one cycle in the labels (which a correct
-// union-find never makes) ends the whole launch within milliseconds and the host reports
-// ISING_ERR_TIMEOUT with the context intact.
+// steps in global memory (about 0.3 s of dependent L2 reads; legitimate walks are far shorter) or
+// kTileSteps in a tile's shared memory (tile_forest.h; a few milliseconds).  A thread that runs out
+// sets the error word, and every loop in global memory gives up as soon as any thread has set it,
+// which it reads every kErrPoll steps.  So one cycle in the labels (which a correct union-find never
+// makes) ends the launch within milliseconds and the host reports ISING_ERR_TIMEOUT with the
+// context intact.
 constexpr int kStepLimit = 1 << 20;
 constexpr int kErrPoll = 64;
 
@@ -152,36 +154,10 @@ __device__ __forceinline__ int8_t colour1_spin(const ClusterArgs& a, long long m
     return a.c[1][mrow * a.pitch + (m - mrow * a.lh)];
 }
 
-// Shared-memory union-find of one tile (same rules as the global one).  A union or a root walk may
-// take kStepLimit steps, a few tens of milliseconds in shared memory; a thread that runs out sets
-// the error word.
-__device__ __forceinline__ int tile_find(volatile int* lab, int x, int& left)
-{
-    while (--left >= 0) {
-        const int p = lab[x];
-        if (p == x) return x;
-        const int gp = lab[p];
-        if (gp == p) return p;
-        lab[x] = gp;  // path halving
-        x = gp;
-    }
-    return x;
-}
-
-__device__ __forceinline__ int tile_root(const volatile int* lab, int x, int* err)
-{
-    for (int left = kStepLimit; left > 0; --left) {
-        const int p = lab[x];
-        if (p == x) return x;
-        x = p;
-    }
-    atomicExch(err, 1);
-    return x;
-}
-
+// Shared-memory union of one tile (same rules as the global one).
 __device__ __forceinline__ void tile_union(int* lab, int a, int b, int* err)
 {
-    int left = kStepLimit;  // shared by the finds and the retries of this union
+    int left = kTileSteps;  // shared by the finds and the retries of this union
     while (true) {
         a = tile_find(lab, a, left);
         b = tile_find(lab, b, left);
@@ -347,7 +323,9 @@ __global__ void __launch_bounds__(kLocalThreads) sw_local_kernel(const ClusterAr
         if (!in) continue;
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
-            const int root = tile_root(lab, cc * RW + r * W + c, a.err);
+            int left = kTileSteps;
+            const int root = tile_root(lab, cc * RW + r * W + c, left);
+            if (left < 0) atomicExch(a.err, 1);
             const int rc = root >= RW;
             const u32 rl = (u32)(root - rc * RW), rr = fast_div(rl, (u32)W, g.w_magic);
             const int gi = (int)(cc * a.S) + (int)(plane + y0 + r) * a.lh + j0 + c;
