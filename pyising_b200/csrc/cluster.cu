@@ -224,10 +224,11 @@ __device__ __forceinline__ void bond_end(const ClusterArgs& a, int k, int y, int
 // bonds that stay in the tile (shared memory) and writes every tile site's label: the global index
 // of its tile-local root.
 //
-// A warp takes a row of the tile, lane c the sites of position c of both colours.  The row's
-// horizontal bonds form runs of a chain; ballots of the two bonds of each colour-0 site give every
+// A warp takes a row of the tile (tiles narrower than a warp: as many rows as fit), a lane the sites
+// of one position of both colours.  The row's horizontal bonds form runs of a chain; ballots of the two bonds of each colour-0 site give every
 // site its run's smallest site as parent at once, without a union.  The vertical bonds then unite
-// runs, once per pair of runs and row (a match over the warp picks one lane of each pair).  Near
+// runs, once per pair of runs and row (a match over the warp picks one lane of each pair), and so do
+// the bonds around the lattice where a tile holds its whole width or height.  Near
 // T_c, where most sites of a tile are in one cluster, one union per bond had long walks and many
 // failed compare-and-swaps.  Measured on one B200, equilibrated at T_c, this kernel 91 -> 30 us at
 // 1024^2, the unions between tiles 37 -> 15 us, whole updates 141 -> 58 us at 1024^2 and 1588 ->
@@ -244,11 +245,18 @@ __global__ void __launch_bounds__(kLocalThreads) sw_local_kernel(const ClusterAr
     const int rn = a.ly - y0 < R ? a.ly - y0 : R;  // rows of this tile
     const int wn = a.lh - j0 < W ? a.lh - j0 : W;  // positions per row of this tile
     unsigned char* masks = reinterpret_cast<unsigned char*>(lab + 2 * RW);
-    const int c = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
-    const int nwarps = (int)(blockDim.x >> 5);
-    const bool in = c < wn;
+    // lanes per row: the least power of two from wn on; 1 << up rows per warp, this lane's the sub-th
+    const int up = wn > 16 ? 0 : wn > 8 ? 1 : wn > 4 ? 2 : 3;
+    const int lane = (int)(threadIdx.x & 31u), c = lane & ((32 >> up) - 1);
+    const int base = lane - c, sub = lane >> (5 - up);
+    const u32 below = (1u << base) - 1u;                       // the lanes of the warp's rows before
+    const u32 inside = ((1u << (wn - 1)) - 1u) << base;        // of this row's sites but the last
+    const int first = ((int)(threadIdx.x >> 5) << up), step_r = (int)(blockDim.x >> 5) << up;
+    const bool wrap_x = g.tx == 1, wrap_y = g.ty == 1;         // the tile reaches around the lattice
     const long long plane = (long long)z * a.ly;
-    for (int r = warp; r < rn; r += nwarps) {
+    for (int rw = first; rw < rn; rw += step_r) {  // (the same for all lanes of a warp)
+        const int r = rw + sub;
+        const bool in = c < wn && r < rn;
         const int y = y0 + r, j = j0 + c;
         const int par = (y + z) & 1;  // 1: the row's other horizontal neighbour is at j + 1
         // the spins the row's bonds join: its own, the opposite colour's of the rows y, y + 1, y - 1
@@ -257,7 +265,7 @@ __global__ void __launch_bounds__(kLocalThreads) sw_local_kernel(const ClusterAr
         const long long row = plane + y;
         const int8_t* c1 = a.c[1] + row * a.pitch;
         const int s1 = in ? c1[j] : 0;
-        int side = __shfl_sync(0xFFFFFFFFu, s1, par ? c + 1 : c - 1);
+        int side = __shfl_sync(0xFFFFFFFFu, s1, par ? lane + 1 : lane - 1);
         unsigned mask = 0;
         if (in) {
             if (par ? c + 1 == wn : c == 0)
@@ -265,11 +273,11 @@ __global__ void __launch_bounds__(kLocalThreads) sw_local_kernel(const ClusterAr
             const u32 q = (u32)row * (u32)a.lh + (u32)j;  // < 2^30
             const int s = a.c[0][row * a.pitch + j];
             const long long step = a.pitch, wrap = (long long)(a.ly - 1) * a.pitch;
-            const int up = c1[(y + 1 == a.ly ? -wrap : step) + j];
+            const int above = c1[(y + 1 == a.ly ? -wrap : step) + j];
             const int dn = c1[(y == 0 ? wrap : -step) + j];
             const u32x4 r0 = philox4x32_10(q, a.t, kBondTag, 0u, a.k0, a.k1);
             mask = (r0.x < a.p_bond && s1 == s ? 1u : 0u) | (r0.y < a.p_bond && side == s ? 2u : 0u) |
-                   (r0.z < a.p_bond && up == s ? 4u : 0u) | (r0.w < a.p_bond && dn == s ? 8u : 0u);
+                   (r0.z < a.p_bond && above == s ? 4u : 0u) | (r0.w < a.p_bond && dn == s ? 8u : 0u);
             if (a.ndim == 3) {
                 const u32x4 r1 = philox4x32_10(q, a.t, kBondTag, 1u, a.k0, a.k1);
                 const long long pl = (long long)a.ly * a.pitch, zwrap = (a.lz - 1) * pl;
@@ -285,42 +293,57 @@ __global__ void __launch_bounds__(kLocalThreads) sw_local_kernel(const ClusterAr
         const bool inner = par ? c + 1 < wn : c > 0;
         const u32 m0 = __ballot_sync(0xFFFFFFFFu, mask & 1u);
         const u32 m1 = __ballot_sync(0xFFFFFFFFu, inner && (mask & 2u) != 0);
-        // bit c: colour-0 site c is in one run with colour-0 site c + 1
-        const u32 link = par ? m1 & (m0 >> 1) : m0 & (m1 >> 1);
-        auto run_start = [&](int at) {  // first colour-0 site of the run of colour-0 site `at`
-            const u32 breaks = ~link & ((1u << at) - 1u);
-            return 32 - __clz((int)breaks);  // 0 without a break
+        // bit of lane l: its colour-0 site is in one run with that of lane l + 1 (in the same row)
+        const u32 link = (par ? m1 & (m0 >> 1) : m0 & (m1 >> 1)) & inside;
+        auto run_start = [&](int at) {  // position of the first colour-0 site of the run of lane `at`
+            const u32 breaks = ~link & ((1u << at) - 1u) & ~below;
+            return max(32 - __clz((int)breaks), base) - base;  // 0 without a break
         };
         if (in) {
             const int i0 = r * W, i1 = RW + r * W + c;
-            lab[i0 + c] = i0 + run_start(c);
+            lab[i0 + c] = i0 + run_start(lane);
             int parent = i1;
-            if ((m0 >> c) & 1u) parent = i0 + run_start(c);
-            else if (par && c > 0 && ((m1 >> (c - 1)) & 1u)) parent = i0 + run_start(c - 1);
-            else if (!par && c + 1 < wn && ((m1 >> (c + 1)) & 1u)) parent = i0 + run_start(c + 1);
+            if ((m0 >> lane) & 1u) parent = i0 + run_start(lane);
+            else if (par && c > 0 && ((m1 >> (lane - 1)) & 1u)) parent = i0 + run_start(lane - 1);
+            else if (!par && c + 1 < wn && ((m1 >> (lane + 1)) & 1u))
+                parent = i0 + run_start(lane + 1);
             lab[i1] = parent;
         }
     }
     __syncthreads();
     volatile int* vlab = lab;
-    for (int r = warp; r < rn; r += nwarps) {
+    for (int rw = first; rw < rn; rw += step_r) {
+        const int r = rw + sub;
+        const bool in = c < wn && r < rn;
         const unsigned mask = in ? masks[r * W + c] : 0u;
-#pragma unroll
-        for (int k = 2; k < 4; ++k) {  // y + 1, y - 1
-            const int nr = k == 2 ? r + 1 : r - 1;
-            const bool active = nr >= 0 && nr < rn && ((mask >> k) & 1u) != 0;
+        // y + 1, y - 1, and around the row
+        for (int k = 2; k < (wrap_x ? 5 : 4); ++k) {
+            int nr = r, nc = c;
+            bool active = ((mask >> (k == 4 ? 1 : k)) & 1u) != 0;
+            if (k == 2) {
+                nr = r + 1 < rn ? r + 1 : 0;
+                active = active && (r + 1 < rn || wrap_y);
+            } else if (k == 3) {
+                nr = r > 0 ? r - 1 : rn - 1;
+                active = active && (r > 0 || wrap_y);
+            } else {
+                const int par = (y0 + r + z) & 1;
+                nc = par ? 0 : wn - 1;
+                active = active && c == wn - 1 - nc;
+            }
             const u32 act = __ballot_sync(0xFFFFFFFFu, active);
             if (active) {
-                const int u = vlab[r * W + c], v = vlab[RW + nr * W + c];
+                const int u = vlab[r * W + c], v = vlab[RW + nr * W + nc];
                 const u32 peers = __match_any_sync(act, (u32)u << 16 | (u32)v);
-                if (c == __ffs((int)peers) - 1) tile_union(lab, u, v, a.err);
+                if (lane == __ffs((int)peers) - 1) tile_union(lab, u, v, a.err);
             }
             __syncwarp();
         }
     }
     __syncthreads();
-    for (int r = warp; r < rn; r += nwarps) {
-        if (!in) continue;
+    for (int rw = first; rw < rn; rw += step_r) {
+        const int r = rw + sub;
+        if (c >= wn || r >= rn) continue;
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
             int left = kTileSteps;
@@ -379,8 +402,9 @@ __global__ void sw_bond_kernel(const ClusterArgs a)
 __global__ void __launch_bounds__(256) sw_cross_kernel(const ClusterArgs a, const TileGeo g)
 {
     const long long lh = a.lh, ly = a.ly, lz = a.lz;
-    const long long per_rows = (long long)g.ty * lz * lh;  // seams between tile rows, per direction
-    const long long per_cols = (long long)g.tx * a.rows;
+    // (a single tile row or column has no seam: its tiles unite the bonds around the lattice too)
+    const long long per_rows = g.ty > 1 ? (long long)g.ty * lz * lh : 0;  // per direction
+    const long long per_cols = g.tx > 1 ? (long long)g.tx * a.rows : 0;
     const long long end_rows = 2 * per_rows, end_cols = end_rows + per_cols;
     const long long n = end_cols + (a.ndim == 3 ? 2 * a.S : 0);
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -569,7 +593,8 @@ static int cluster_step(ising_sim* h, u32 t, u64 seed, u32 p_bond, bool flip)
         // eight, 256^2 43 / 35 us)
         const int threads = tiles >= 4 * h->sm_count ? kLocalThreads / 2 : kLocalThreads;
         sw_local_kernel<<<(unsigned)tiles, threads, smem, h->stream>>>(a, g);
-        sw_cross_kernel<<<grid, 256, 0, h->stream>>>(a, g);
+        if (g.tx > 1 || g.ty > 1 || h->ndim == 3)  // else one tile holds the lattice
+            sw_cross_kernel<<<grid, 256, 0, h->stream>>>(a, g);
     } else {
         sw_init_kernel<<<grid, 256, 0, h->stream>>>(a.label, 2 * a.S);
         sw_bond_kernel<<<grid, 256, 0, h->stream>>>(a);
