@@ -398,18 +398,22 @@ __global__ void sw_bond_kernel(const ClusterArgs a)
 // tile rows (the last one around the lattice) at each position, the one bond across every seam
 // between tile columns at each row, and in 3D the two z bonds of every colour-0 site.  Lanes run
 // along a seam, where neighbouring bonds mostly join the same two tile clusters: one lane per pair
-// of labels in a warp does the union.
-__global__ void __launch_bounds__(256) sw_cross_kernel(const ClusterArgs a, const TileGeo g)
+// of labels in a warp does the union.  A thread takes `parts` z bonds one after another: the rows of
+// two tiles in neighbouring planes mostly join the same two clusters, too, and in an ordered lattice
+// those unions get in each other's way when all of them start at once (cluster_z_parts).
+__global__ void __launch_bounds__(256) sw_cross_kernel(const ClusterArgs a, const TileGeo g, int parts)
 {
     const long long lh = a.lh, ly = a.ly, lz = a.lz;
     // (a single tile row or column has no seam: its tiles unite the bonds around the lattice too)
     const long long per_rows = g.ty > 1 ? (long long)g.ty * lz * lh : 0;  // per direction
     const long long per_cols = g.tx > 1 ? (long long)g.tx * a.rows : 0;
     const long long end_rows = 2 * per_rows, end_cols = end_rows + per_cols;
-    const long long n = end_cols + (a.ndim == 3 ? 2 * a.S : 0);
+    const long long begin_z = (end_cols + 31) / 32 * 32, z_part = 2 * a.S / parts;  // S % 4 == 0
+    const long long n = a.ndim == 3 ? begin_z + z_part : end_cols;
     const long long stride = (long long)gridDim.x * blockDim.x;
     const int lane = (int)(threadIdx.x & 31u);
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i - lane < n; i += stride) {
+    int part = 0;  // of the z bonds; the same for all lanes of a warp
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i - lane < n;) {
         long long q = -1, m = 0;  // colour-0 and colour-1 positions of the bond
         int k = 0;
         if (i < end_rows) {
@@ -434,9 +438,10 @@ __global__ void __launch_bounds__(256) sw_cross_kernel(const ClusterArgs a, cons
             k = 1;
             q = row * lh + (par ? last : next);
             m = row * lh + (par ? next : last);
-        } else if (i < n) {
-            const int up = i - end_cols >= a.S;
-            q = i - end_cols - up * a.S;
+        } else if (i >= begin_z && i < n) {
+            const long long bond = i - begin_z + part * z_part;
+            const int up = bond >= a.S;
+            q = bond - up * a.S;
             k = up ? 5 : 4;
             const long long pl = ly * lh;
             const long long z = (u32)q / (u32)pl;
@@ -450,6 +455,9 @@ __global__ void __launch_bounds__(256) sw_cross_kernel(const ClusterArgs a, cons
             if (lane == __ffs((int)peers) - 1) uf_union(a.label, u, v, a.err);
         }
         __syncwarp();
+        if (i - lane >= begin_z && ++part < parts) continue;
+        part = 0;
+        i += stride;
     }
 }
 
@@ -553,6 +561,15 @@ static int cluster_tiles(const ising_sim* h, TileGeo* g)
     return g->tx * g->ty * h->lz;
 }
 
+// z bonds per thread of the unions between tiles.  Four in lattices whose z bonds would all start at
+// once and that are well ordered (3D bonds are critical at p = 0.358): one B200, us per update, one /
+// four: 8x8x4096 at beta 0.28 165 / 75, 64^3 125 / 80, 16x16x1024 157 / 82; but at the critical beta
+// 38 / 48, 42 / 51, 40 / 49, and 128^3 at 0.28 363 / 701.
+static int cluster_z_parts(const ClusterArgs& a, int threads)
+{
+    return a.ndim == 3 && a.p_bond >= 0x66666666u && 2 * a.S <= threads ? 4 : 1;
+}
+
 static unsigned char* cluster_masks(ising_sim* h, long long S)
 {
     return reinterpret_cast<unsigned char*>(h->d_label) + 2 * S * sizeof(int) + 256;
@@ -594,7 +611,7 @@ static int cluster_step(ising_sim* h, u32 t, u64 seed, u32 p_bond, bool flip)
         const int threads = tiles >= 4 * h->sm_count ? kLocalThreads / 2 : kLocalThreads;
         sw_local_kernel<<<(unsigned)tiles, threads, smem, h->stream>>>(a, g);
         if (g.tx > 1 || g.ty > 1 || h->ndim == 3)  // else one tile holds the lattice
-            sw_cross_kernel<<<grid, 256, 0, h->stream>>>(a, g);
+            sw_cross_kernel<<<grid, 256, 0, h->stream>>>(a, g, cluster_z_parts(a, grid * 256));
     } else {
         sw_init_kernel<<<grid, 256, 0, h->stream>>>(a.label, 2 * a.S);
         sw_bond_kernel<<<grid, 256, 0, h->stream>>>(a);
