@@ -21,7 +21,9 @@ events on the simulation's stream) by coordinate descent from the defaults, and 
 configuration in a JSON cache (``$PYISING_B200_TUNE_CACHE``, else
 ``~/.cache/pyising_b200/tune.json``) keyed by the GPU, variant, algorithm and shape.  New
 simulations pick up a cached configuration automatically (:func:`apply_cached`); with
-``PYISING_B200_AUTOTUNE=1`` a shape without one is tuned on first use.
+``PYISING_B200_AUTOTUNE=1`` a shape without one is tuned on first use.  An entry belongs to the
+kernels and automatic schedules that it was measured with (:data:`SCHEDULES`): entries of other
+ones, whose knobs may now select a slower path than the default, are not applied.
 
 The reference has no counterpart: its CUDA kernels use one fixed launch shape
 (src/pyising/backends/cupy_backend.py:68-72,129-135).
@@ -44,6 +46,10 @@ KNOBS = {"band": 1, "chunk_width": 2, "blocks_per_sm": 3, "msc_waves": 4, "graph
          "msc_kernel": 9}
 DEFAULTS = {"band": 0, "chunk_width": 16, "blocks_per_sm": 8, "msc_waves": 1, "graph_chunk": 32,
             "msc_kernel": 0, "schedule": "auto"}
+
+#: Generation of the kernels and automatic schedules, stored with every cache entry; raised when
+#: they change so that a configuration measured before may no longer be the best.
+SCHEDULES = 2
 
 _lock = threading.Lock()
 _cache_mem: dict[Path, dict] = {}  # cache file contents by path, read once per process
@@ -85,12 +91,12 @@ def search_space(variant: str, shape, algorithm: str = "metropolis") -> dict[str
         space["msc_kernel"] = [0, 1] + ([2, 3, 4, 5, 6, 7] if (lh // 64) % 32 == 0 else [])
         space["msc_waves"] = [1, 2, 4]
     space["blocks_per_sm"] = [8, 4, 16]
-    if variant == "int8" and len(shape) == 2:
-        space["schedule"] = ["auto", "launches", "persistent"]
-        if lh % 16 == 0 and shape[0] % 8 == 0 and shape[0] >= 16 and 32 * lh <= 96 * 1024:
-            space["schedule"].append("temporal")
-    else:
-        space["schedule"] = ["auto", "launches"]
+    space["schedule"] = ["auto", "launches"]
+    if len(shape) == 2:
+        if variant == "int8":
+            space["schedule"].append("persistent")
+        # 2D tiles (single half-sweeps where the rows do not fit a tile)
+        space["schedule"].append("temporal")
     space["graph_chunk"] = [32, 8, 128]
     return space
 
@@ -113,11 +119,12 @@ def load_cache(path: Path | None = None) -> dict[str, dict]:
 
 
 def save_entry(k: str, entry: dict, path: Path | None = None) -> None:
-    """Adds one entry to the cache file (read-modify-write, replaced atomically)."""
+    """Adds one entry, stamped with :data:`SCHEDULES`, to the cache file (read-modify-write, replaced
+    atomically)."""
     p = Path(path) if path is not None else cache_path()
     with _lock:
         data = _read(p)
-        data[k] = entry
+        data[k] = dict(entry, schedules=SCHEDULES)
         p.parent.mkdir(parents=True, exist_ok=True)
         tmp = p.with_suffix(p.suffix + f".{os.getpid()}.tmp")
         tmp.write_text(json.dumps(data, indent=1, sort_keys=True))
@@ -127,7 +134,9 @@ def save_entry(k: str, entry: dict, path: Path | None = None) -> None:
 
 def lookup(k: str, path: Path | None = None) -> dict | None:
     entry = load_cache(path).get(k)
-    return entry.get("config") if isinstance(entry, dict) else None
+    if not isinstance(entry, dict) or entry.get("schedules") != SCHEDULES:
+        return None
+    return entry.get("config")
 
 
 # ------------------------------------------------------------------------- knobs -----------
