@@ -137,7 +137,9 @@ int ising_set_schedule(ising_sim* h, int schedule, int test_mute_band);
  *   ISING_KNOB_BAND           int8: rows of one plane a thread walks, reusing the opposite
  *                             colour's rows (halo depth); 0 = occupancy-based default
  *   ISING_KNOB_CHUNK_WIDTH    int8: bytes (4 sites each per 32-bit word) per thread: 16, 8, 4
- *   ISING_KNOB_BLOCKS_PER_SM  grid cap in blocks of 256 threads per SM (default 8)
+ *   ISING_KNOB_BLOCKS_PER_SM  grid cap in blocks of 256 threads per SM of the kernels that walk
+ *                             bands of rows (default 8); no effect on tiles, on the smaller int8
+ *                             lattices that run one chunk per thread, and on packed sweeps
  *   ISING_KNOB_MSC_WAVES      msc: warp ranges per resident warp (default 1)
  *   ISING_KNOB_GRAPH_CHUNK    sweeps per captured graph of an unmeasured run (default 32) */
 #define ISING_KNOB_BAND 1

@@ -6,7 +6,8 @@ by site, sweep and colour, and every schedule visits the same sites with the sam
 * ``band``          int8: rows of one plane a thread walks while the opposite colour's rows
                     slide through its registers (the halo reuse depth); 0 = occupancy default;
 * ``chunk_width``   int8: bytes per thread and row, 16, 8 or 4 (4, 2 or 1 words of 4 sites);
-* ``blocks_per_sm`` grid size in blocks of 256 threads per SM;
+* ``blocks_per_sm`` grid size in blocks of 256 threads per SM of the int8 kernels that walk bands (no
+                    effect on tiles and on small lattices, which run one chunk per thread);
 * ``msc_kernel``    msc: schedule: automatic, word ranges per warp, or 32-word column strips walked
                     down a band of rows with 4 or 3 Philox blocks per word at intake and registers
                     bounded for 2, 3 or 4 resident blocks;

@@ -10,13 +10,16 @@ pytestmark = pytest.mark.gpu
 BETA_C_2D = 0.44068679350977147
 
 
-def second_pair(variant, shape, schedule="auto"):
+def second_pair(variant, shape, schedule="auto", knobs=None):
     """Whether a swept lattice holds a second pair of colour arrays."""
+    from pyising_b200 import autotune
     from pyising_b200.backend import B200Int8, B200MultiSpin
 
     cls = B200MultiSpin if variant == "msc" else B200Int8
     sim = cls(shape, BETA_C_2D, seed=3, init="cold")
     sim.set_schedule(schedule)
+    if knobs:
+        autotune.apply(sim, knobs)
     before = sim.device_bytes()
     sim.sweep(3)
     more = sim.device_bytes() - before
@@ -46,3 +49,14 @@ def test_automatic_schedule_takes_tiles_where_they_are_faster(variant, shape, ti
     if torch.cuda.get_device_properties(0).multi_processor_count != 148:
         pytest.skip("the choice depends on the number of SMs")
     assert second_pair(variant, shape) == tiles
+
+
+def test_launch_knobs_set_by_hand_select_the_half_sweeps_they_belong_to():
+    shape = (1600, 1600)  # above 512K sites per colour
+    assert second_pair("int8", shape)
+    for name, default, value in [("band", 0, 2), ("chunk_width", 16, 4)]:
+        assert second_pair("int8", shape, knobs={name: default})
+        assert not second_pair("int8", shape, knobs={name: value})
+    for name, default, value in [("msc_kernel", 0, 1), ("msc_waves", 1, 2)]:
+        assert second_pair("msc", (256, 1024), knobs={name: default})
+        assert not second_pair("msc", (256, 1024), knobs={name: value})
