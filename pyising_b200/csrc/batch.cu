@@ -979,35 +979,45 @@ private:
         int rc = upload(lats.data(), lats.size() * sizeof(BatchLattice), (void**)&d_lats_, &lats_cap_);
         if (rc == ISING_OK)
             rc = upload(items.data(), items.size() * sizeof(BatchItem), (void**)&d_items_, &items_cap_);
+        if (rc != ISING_OK) return rc;
+        plan_streams();
         dirty_ = false;
-        if (rc == ISING_OK) rc = plan_streams();
-        return rc;
+        return ISING_OK;
     }
 
     // Every class advances on a stream of its own when there are several: their lattices are
     // independent, and a class alone often leaves most of the GPU waiting.  The engine's stream
     // waits for all of them at every sweep (join), they wait for it only after it did something
     // (fork): admissions, results, work lists, graph chunks.
-    int plan_streams()
+    // Without streams or events to be had, all classes stay on the engine's stream.
+    void plan_streams()
     {
-        size_t n = int8_launches_.size() + (msc_one_.empty() ? 0 : 1) + classes_.size();
-        n_aux_ = n > 1 ? n : 0;
-        while (aux_.size() < n_aux_) {
+        const size_t n = int8_launches_.size() + (msc_one_.empty() ? 0 : 1) + classes_.size();
+        forked_ = false;
+        n_aux_ = n > 1 && class_streams(n) ? n : 0;
+    }
+
+    // Makes n class streams and the fork event; whether all of them exist.
+    bool class_streams(size_t n)
+    {
+        if (!fork_event_ &&
+            cudaEventCreateWithFlags(&fork_event_, cudaEventDisableTiming) != cudaSuccess) {
+            fork_event_ = nullptr;
+            cudaGetLastError();
+            return false;
+        }
+        while (aux_.size() < n) {
             Aux a;
             cudaError_t e = cudaStreamCreateWithFlags(&a.stream, cudaStreamNonBlocking);
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&a.event, cudaEventDisableTiming);
             if (e != cudaSuccess) {
                 if (a.stream) cudaStreamDestroy(a.stream);
-                return cuda_fail(e, "batch class stream");
+                cudaGetLastError();
+                return false;
             }
             aux_.push_back(a);
         }
-        if (n_aux_ && !fork_event_) {
-            const cudaError_t e = cudaEventCreateWithFlags(&fork_event_, cudaEventDisableTiming);
-            if (e != cudaSuccess) return cuda_fail(e, "batch fork event");
-        }
-        forked_ = false;
-        return ISING_OK;
+        return true;
     }
 
     // The class streams wait for the engine's.
