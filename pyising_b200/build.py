@@ -25,8 +25,10 @@ BUILD = ROOT / "_build"
 LIB = PKG / "libising_b200.so"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-O3", "--expt-relaxed-constexpr",
-              "-I", str(INCLUDE), "-I", str(CSRC)]
+# Uncompressed device code: the first launch of a kernel of a compressed module waits for the module
+# to be unpacked (the first batch of a process 22 ms, uncompressed 9).
+NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--no-compress", "-Xcompiler", "-fPIC,-O3",
+              "--expt-relaxed-constexpr", "-I", str(INCLUDE), "-I", str(CSRC)]
 
 
 def nvcc() -> str:
