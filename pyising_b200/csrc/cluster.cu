@@ -198,28 +198,6 @@ __device__ __forceinline__ void tile_origin(const ClusterArgs& a, const TileGeo&
     j0 = (rem - by * g.tx) * g.W;
 }
 
-// Colour-1 coordinates (y, j, z) of bond k of colour-0 site (y, j, z) (the order of the bond
-// bits), periodic.
-__device__ __forceinline__ void bond_end(const ClusterArgs& a, int k, int y, int j, int z,
-                                         int& ny, int& nj, int& nz)
-{
-    ny = y;
-    nj = j;
-    nz = z;
-    if (k == 1) {
-        const int par = (y + z) & 1;  // colour 0
-        nj = par ? (j + 1 == a.lh ? 0 : j + 1) : (j == 0 ? a.lh - 1 : j - 1);
-    } else if (k == 2) {
-        ny = y + 1 == a.ly ? 0 : y + 1;
-    } else if (k == 3) {
-        ny = y == 0 ? a.ly - 1 : y - 1;
-    } else if (k == 4) {
-        nz = z + 1 == a.lz ? 0 : z + 1;
-    } else if (k == 5) {
-        nz = z == 0 ? a.lz - 1 : z - 1;
-    }
-}
-
 // Tile b: draws the bonds of the tile's colour-0 sites, stores their masks, unites the active
 // bonds that stay in the tile (shared memory) and writes every tile site's label: the global index
 // of its tile-local root.

@@ -65,7 +65,6 @@ __device__ __forceinline__ u32x4 philox4x32_10(u32 c0, u32 c1, u32 c2, u32 c3, u
 // "spin down" flag, and XOR with 0xFE flips.
 constexpr u32 kBit2 = 0x04040404u;
 constexpr u32 kBit5 = 0x20202020u;
-constexpr u32 kFlip = 0xFEFEFEFEu;
 
 // Sum of the four bytes of v (each byte small and non-negative).
 __device__ __forceinline__ int byte_sum(u32 v) { return (int)__dp4a(v, 0x01010101u, 0u); }
