@@ -720,9 +720,9 @@ int ising_sweep(ising_sim* h, uint64_t t0, int64_t n_sweeps, int64_t measure_eve
     // Small 2D int8 lattices: all sweeps in one persistent cooperative launch.
     const bool persistent_ok = h->variant == ISING_VARIANT_INT8 && h->ndim == 2 &&
                                n_sweeps > 0 && n_sweeps < (1LL << 30);
-    // (The automatic schedule uses graphs: on B200 the per-half-sweep chain of flag, halo
-    // reads and fence of the persistent kernel measured 1.9x slower than replayed graphs at
-    // 1024^2: 141 against 273 flips/ns, and 320 for the temporal tiles.)
+    // (On request only: on B200 the per-half-sweep chain of flag, halo reads and fence of the
+    // persistent kernel is about 3.7 us, 141 flips/ns at 1024^2 against 300 for replayed graphs of
+    // single half-sweeps and 391 for the tiles.)
     const bool want_persistent = h->schedule == ISING_SCHEDULE_PERSISTENT;
     if (persistent_ok && want_persistent) {
         if (!h->d_flags) {

@@ -83,16 +83,16 @@ __global__ void __launch_bounds__(kQueueWarps * 32, MINB)
 
 // Rows of any number of words: lane g of the launch walks the rows of band g / nw in column g % nw,
 // so neighbouring lanes still read neighbouring words and no lane is without a column but at the
-// end.  Bands and rows are even, so every band starts with the same parity.
+// end.  Bands and rows are even, so every band starts with the same parity (lane_plan.h: which).
 //
 // Like the strips it is bound by the integer pipes; against the word ranges it has the levels of
 // two rows in flight per step, keeps the opposite colour's words of the next rows in registers
-// and needs no division or parity selection per word.  Measured on one B200, ranges -> lanes
-// (flips/ns): 4200x4224 1730 -> 2060, 6000x5248 1999 -> 2282, 6144^2 2384 -> 2822, 10000x9984
-// 2787 -> 3216, 20000x20096 3257 -> 4171, 160000x128 1621 -> 2288.  More and shorter bands (two
-// waves of warps) were slower from 5000x4992 on (20000x20096 3961).  Against the strips, which
-// walk rows of whole 32-word strips in the same steps: 4096^2 2115 both, 4600x12288 3083 -> 3155,
-// 8192^2 2971 -> 3038, 16384^2 4022 -> 4085.
+// and needs no division or parity selection per word.  Measured on one B200 with replayed graphs of
+// single half-sweeps, ranges -> lanes (flips/ns): 3072^2 1267 -> 1438, 4200x4224 1722 -> 1945,
+// 6000x5248 1982 -> 2343, 6144^2 2376 -> 2815, 10000x9984 2784 -> 3215, 20000x20096 3257 -> 4182.
+// More and shorter bands (two waves of warps) were slower (20000x20096 3961).  Against the strips,
+// which walk rows of whole 32-word strips in the same steps: 4096^2 1802 -> 1876, 4600x12288
+// 3076 -> 3150, 8192^2 2949 -> 3017, 16384^2 4017 -> 4082.
 template <bool MEAS>
 __global__ void __launch_bounds__(kQueueWarps * 32, 2)
     msc_lane_kernel(const MscHalf p_in, int band, int bands)
