@@ -110,16 +110,21 @@ int ising_half_sweep(ising_sim* h, int color, uint64_t t);
 
 /* How ising_sweep issues its half-sweeps (no counterpart in the reference, which launches one
  * kernel per half-sweep from Python):
- *   ISING_SCHEDULE_AUTO       graphs for whole chunks of sweeps, launches for the rest (the
+ *   ISING_SCHEDULE_AUTO       graphs for whole chunks of sweeps, launches for the rest; the
  *                             temporal tiles below for 2D lattices of up to 6.5M int8 or 16M
- *                             packed sites per colour);
+ *                             packed sites per colour where they are faster (not for lattices
+ *                             much wider than high);
  *   ISING_SCHEDULE_LAUNCHES   one kernel launch per half-sweep;
  *   ISING_SCHEDULE_GRAPHS     replayed CUDA graphs of whole chunks of sweeps;
  *   ISING_SCHEDULE_PERSISTENT one cooperative launch for all sweeps (2D int8; others fall back):
  *                             bands of rows wait only for their neighbours, every wait bounded;
  *   ISING_SCHEDULE_TEMPORAL   launches that each run several half-sweeps on
  *                             shared-memory tiles with recomputed halos (2D lattices whose
- *                             rows fit; others fall back).
+ *                             rows fit; others fall back).  The calling thread issues every
+ *                             launch, one per 3 to 16 half-sweeps (a graph holds 64): a sweep
+ *                             call returns before the device is done, but not long before.  A
+ *                             program whose host thread has other work meanwhile, or that
+ *                             drives many lattices from many threads, can choose GRAPHS.
  * All schedules give identical results.  test_mute_band >= 0 makes that band of a persistent
  * run stop publishing its progress, so its neighbours' bounded waits expire: the sweep then
  * reports ISING_ERR_TIMEOUT (the lattice is no longer valid); pass -1 otherwise. */

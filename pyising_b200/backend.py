@@ -135,7 +135,9 @@ class _B200Simulation(IsingSimulation):
         """How sweeps are issued: ``"auto"``, ``"launches"`` (one kernel per half-sweep),
         ``"graphs"`` (replayed CUDA graphs), ``"persistent"`` (one cooperative launch for all
         sweeps; 2D int8) or ``"temporal"`` (launches that each run several half-sweeps on
-        shared-memory tiles; 2D lattices).  Results are identical.  ``test_mute_band`` >= 0 is a
+        shared-memory tiles; 2D lattices).  Results are identical.  The tiles, which ``"auto"``
+        takes for small 2D lattices, are launched one by one from the calling thread, which they
+        keep busy for most of the run; ``"graphs"`` returns at once.  ``test_mute_band`` >= 0 is a
         test hook that makes one band of a persistent run stop publishing, so the run reports a
         time-out."""
         check(lib().ising_set_schedule(self._h, self.SCHEDULES[schedule], int(test_mute_band)),

@@ -21,8 +21,8 @@
 // A step is bound by the latency of one warp's chain of instructions (draws, barrier, neighbour
 // loads, decisions, store), not by a pipe: about 0.5 us (int8) to 0.8 us (msc) on lattices whose
 // rows are a few words.  Measured on one B200, flips/ns, single half-sweeps -> tiles: int8 256^2
-// 26 -> 48, 1024^2 303 -> 371, 2048^2 640 -> 680; msc 256^2 13 -> 41, 1152^2 236 -> 530, 2048^2
-// 728 -> 1212, 4096^2 1750 -> 2043.
+// 26 -> 51, 1024^2 300 -> 391, 2048^2 646 -> 700; msc 512^2 52 -> 156, 1152^2 239 -> 570, 2048^2
+// 742 -> 1267, 4096^2 1861 -> 2116.  tile_plan.h: bands, depths and where tiles pay.
 #include <cstring>
 
 #include "capi_internal.h"
