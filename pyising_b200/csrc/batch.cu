@@ -163,7 +163,8 @@ __device__ __forceinline__ void batch_int8_slots(const Int8Half& p, const Int8De
         }
         const int y0 = yb * L.band;
         const int y1 = y0 + L.band < L.ly ? y0 + L.band : L.ly;
-        int8_band<V, NDIM, RULE, MIXED, MEAS>(p, z, y0, y1, j0, rt, m_acc, e_acc);
+        int8_band<V, NDIM, RULE, MIXED, MEAS, NDIM == 2 || kRowPairs<RULE, MIXED, MEAS>>(
+            p, z, y0, y1, j0, rt, m_acc, e_acc);
     }
 }
 

@@ -377,8 +377,12 @@ __device__ __forceinline__ void int8_band_row(const Int8Half& p, const BandRow& 
 // are on, is then fixed in the code, and the sliding rows are renamed every second row only.  Not
 // so padded rows that are updated and measured: two such rows in flight need more than the 64
 // registers of four blocks per SM (spilled, a measured sweep of 3D 300x300x304 took 58.4 us, row by
-// row 44.7).
-template <int V, int NDIM, int RULE, bool MIXED, bool MEAS>
+// row 44.7).  (PAIRS: batches have measured and unmeasured rows in one kernel.)
+template <int RULE, bool MIXED, bool MEAS>
+constexpr bool kRowPairs = !(MIXED && MEAS && RULE != kObserve);
+
+template <int V, int NDIM, int RULE, bool MIXED, bool MEAS,
+          bool PAIRS = kRowPairs<RULE, MIXED, MEAS>>
 __device__ __forceinline__ void int8_band(const Int8Half& p, int z, int y0, int y1, int j0,
                                           const u32* rt, long long& m_acc, long long& e_acc)
 {
@@ -426,7 +430,7 @@ __device__ __forceinline__ void int8_band(const Int8Half& p, int z, int y0, int 
             c = d2;
         }
     };
-    if constexpr (!(MIXED && MEAS && RULE != kObserve)) {
+    if constexpr (PAIRS) {
         if (((y0 | y1) & 1) == 0) {
             if (par0) pairs(std::integral_constant<int, 1>{});
             else pairs(std::integral_constant<int, 0>{});
