@@ -26,4 +26,15 @@ inline int int8_default_band(long long rows, int ly, int cpr, int sm_count)
     return b;
 }
 
+// Longest band of batched half-sweeps for a lattice of rows of `cpr` chunks, whatever the class has to
+// spare: in rows of one chunk (see above) four rows, in 3D two, and in 3D bands of 8 rows pay from 16
+// chunks on only.  Measured on one B200, us, bands of 8 -> this: 3D heat bath 6 x 1000x1000x24 8006 ->
+// 4509, 4 x 2000x2000x32 4000 -> 2698, 4 x 300x300x304 3235 -> 2817, 2 x 400x400x416 3058 -> 2687; 2D 4 x
+// 2000000x32 2880 -> 2115; and bands of 4 -> 8: 2 x 512^3 2333 -> 2239, 4 x 100x1000x1000 3859 -> 3720.
+inline int int8_band_limit(int ndim, int cpr)
+{
+    if (cpr == 1) return ndim == 3 ? 2 : 4;
+    return ndim == 3 && cpr < 16 ? 4 : 64;
+}
+
 }  // namespace ising

@@ -26,6 +26,7 @@
 #include <thread>
 #include <vector>
 
+#include "band_plan.h"
 #include "capi_internal.h"
 #include "int8_core.cuh"
 #include "msc_core.cuh"
@@ -912,7 +913,7 @@ private:
                 }
                 Int8Launch& P = launches.back();
                 Int8Desc D = kv.second[i];
-                D.band = band < D.ly ? band : D.ly;
+                D.band = std::min(std::min(band, int8_band_limit(kc.ndim, D.cpr)), D.ly);
                 D.bpp = (D.ly + D.band - 1) / D.band;
                 const long long nslots = (long long)D.lz * D.bpp * D.cpr;
                 D.nslots = (int)nslots;

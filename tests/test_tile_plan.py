@@ -32,6 +32,7 @@ extern "C" int band(long long rows, int ly, int cpr, int sms)
 {
     return ising::int8_default_band(rows, ly, cpr, sms);
 }
+extern "C" int limit(int ndim, int cpr) { return ising::int8_band_limit(ndim, cpr); }
 extern "C" int plan(int msc, int ly, int units, int row_bytes, int sms, int* shape, double* us)
 {
     const ising::TileRows r{msc != 0, ly, units, (size_t)row_bytes, sms};
@@ -153,3 +154,9 @@ def test_default_band(plan, shape, best):
         rows *= extent
     got = plan.band(ctypes.c_longlong(rows), shape[-2], -(-shape[-1] // 32), 148)
     assert got in best
+
+
+@pytest.mark.parametrize("ndim,cpr,most", [(2, 1, 4), (2, 2, 64), (2, 512, 64), (3, 1, 2), (3, 2, 4),
+                                           (3, 15, 4), (3, 16, 64)])
+def test_band_limit_of_batches(plan, ndim, cpr, most):
+    assert plan.limit(ndim, cpr) == most
