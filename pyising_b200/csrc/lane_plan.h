@@ -18,11 +18,13 @@ constexpr int kLaneWords = 256;
 // bands of 16, 32 or 48 rows were slower than the next larger ones (1076018x128 2698, word ranges
 // 2994).
 //
-// Bands come in pairs of rows, so short bands may leave many lanes without one.  Word ranges are
-// then faster (flips/ns, ranges / lanes): bands of 4 rows from 51% of the lanes 1549 / 1506
-// (2402x8192), from 75% 2256 / 2177 (3552x8192), from 97% 2435 / 2812; bands of 6 from 67% 2143 /
-// 2211 (4794x8192).  Bands of 2 are faster from half the lanes and less (650x8192 737 / 824).  Rows of
-// more words than lanes leave no band height at all.
+// Bands come in pairs of rows, so short bands may leave many lanes without one, where word ranges,
+// in steps of 32 words per warp, waste less.  With one wave of either, a half-sweep takes about 2.45 us
+// + 1.09 per row of a band, or 2.2 us + 1.4 per word of a lane's share (flips/ns, ranges / lanes): bands
+// of 4 rows for 2.03 words per lane 1549 / 1506 (2402x8192), for 3 2256 / 2177 (3552x8192), for 3.1 1896
+// / 2172 (58726x512), for 3.9 2435 / 2812; bands of 6 for 4.05 2143 / 2211 (4794x8192).  Bands of 2 are
+// always faster (650x8192 737 / 824, 1242x8192 1024 / 1143).  Rows of more words than lanes leave no
+// band height at all.
 inline long long lane_band(long long rows, long long nw, long long lanes, long long sms)
 {
     const long long words = rows * nw;
@@ -32,7 +34,8 @@ inline long long lane_band(long long rows, long long nw, long long lanes, long l
     if (band > rows) band = rows;
     while (band < rows && (rows + band - 1) / band * nw > lanes) band += 2;
     if (nw == 1 && band % 16 == 0 && band < rows) band += 2;
-    if (band > 2 && (nw > lanes || 5 * words < lanes * 2 * (band + 4))) return 0;
+    const long long share = (words + lanes - 1) / lanes;
+    if (band > 2 && (nw > lanes || 220 + 140 * share < 245 + 109 * band)) return 0;
     return band;
 }
 

@@ -122,7 +122,7 @@ def test_lane_bands_fit_the_resident_lanes(plan, nw, fill):
         assert band == 0
         return
     assert band % 2 == 0 and 0 <= band <= rows
-    if nw <= 128 and not 2 < words / LANES < 3.3:
+    if nw <= 128 and not 2 < words / LANES <= 4:
         assert band > 0  # word ranges only where the walk would leave many lanes idle
     if band > 2:
         assert -(-rows // band) * nw <= LANES  # one wave: no block left over
@@ -130,7 +130,7 @@ def test_lane_bands_fit_the_resident_lanes(plan, nw, fill):
         assert words >= 0.4 * LANES * band  # and not mostly idle
 
 
-@pytest.mark.parametrize("shape,band", [((505172, 384), 22), ((2402, 8192), 0), ((3552, 8192), 0),
+@pytest.mark.parametrize("shape,band", [((505172, 384), 22), ((2402, 8192), 0), ((3552, 8192), 0), ((58726, 512), 4), ((302, 128000), 0),
                                         ((4616, 8192), 4), ((4794, 8192), 6), ((650, 8192), 2),
                                         ((4600, 4608), 0), ((6000, 5248), 4), ((16384, 16384), 28),
                                         ((1152, 1152), 0)], ids=str)
