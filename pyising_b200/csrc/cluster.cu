@@ -540,12 +540,14 @@ static int cluster_tiles(const ising_sim* h, TileGeo* g)
 }
 
 // z bonds per thread of the unions between tiles.  Four in lattices whose z bonds would all start at
-// once and that are well ordered (3D bonds are critical at p = 0.358): one B200, us per update, one /
-// four: 8x8x4096 at beta 0.28 165 / 75, 64^3 125 / 80, 16x16x1024 157 / 82; but at the critical beta
-// 38 / 48, 42 / 51, 40 / 49, and 128^3 at 0.28 363 / 701.
+// once, that are well ordered (3D bonds are critical at p = 0.358) and not too small to profit: one
+// B200, us per update, one / four: at beta 0.28 8x8x4096 165 / 75, 64^3 125 / 80, 16x16x1024 157 / 82,
+// 48^3 88 / 65; but 128x16x16 43 / 48, 128^3 363 / 701, and at the critical beta 8x8x4096 38 / 48, 64^3
+// 42 / 51.
 static int cluster_z_parts(const ClusterArgs& a, int threads)
 {
-    return a.ndim == 3 && a.p_bond >= 0x66666666u && 2 * a.S <= threads ? 4 : 1;
+    const bool fits = 2 * a.S <= threads && 6 * a.S >= threads;
+    return a.ndim == 3 && a.p_bond >= 0x66666666u && fits ? 4 : 1;
 }
 
 static unsigned char* cluster_masks(ising_sim* h, long long S)

@@ -51,3 +51,19 @@ def test_updates_are_those_of_one_union_find(shape):
     for series, lattice in out[1:]:
         np.testing.assert_array_equal(series, out[0][0])
         np.testing.assert_array_equal(lattice, out[0][1])
+
+
+@pytest.mark.parametrize("shape", [(48, 48, 48), (4, 40, 1024)], ids=str)
+def test_unions_of_several_planes_bonds_per_thread(shape):
+    """Ordered 3D lattices of a size at which a thread takes four z bonds."""
+    from pyising_b200.backend import B200Int8
+
+    out = []
+    for tile in (1, 0, 1000):
+        sim = B200Int8(shape, 0.3, seed=9, init="hot")
+        set_cluster_tile(sim, tile)
+        out.append((sim.cluster_sweep(4, measure=True), sim.cluster_labels(step=2)))
+    for series, (labels, bonds) in out[1:]:
+        np.testing.assert_array_equal(series, out[0][0])
+        np.testing.assert_array_equal(labels, out[0][1][0])
+        np.testing.assert_array_equal(bonds, out[0][1][1])
