@@ -5,14 +5,14 @@
 // band is `band` consecutive rows of one plane.  A thread takes slots grid-stride and walks its
 // band's rows top to bottom (int8_band), so consecutive threads of a warp read consecutive
 // 16-byte chunks of the same rows.  Longer bands reuse more opposite-colour rows but leave fewer
-// slots to fill the GPU; the launcher's default picks the longest band (up to 16 rows) that
-// still gives every SM a wave of resident threads, and a tuned value can replace it.
+// slots to fill the GPU; the launcher's default (band_plan.h) weighs the two, and a tuned value can
+// replace it.
 //
 // The band walk is bound by the logic (ALU) pipe: two cycles per warp and SM quarter for each
 // logic, compare, permute or shift instruction, and two more for each wide multiply of the random
 // numbers (which also takes four of the multiplier pipe).  A 16-site chunk takes about 205 such
-// slots (258 before the decisions became lookups); byte cuts (dp4a), predicated adds and sums run
-// on the multiplier pipe, which they fill to 82%.  Measured on one B200, flips/ns before -> after:
+// slots (258 before the decisions became lookups), by that count 86% of the time; byte cuts (dp4a),
+// predicated adds and sums run on the multiplier pipe (busy 77% in ncu).  Measured on one B200, flips/ns before -> after:
 // 2D 16384^2 1030 -> 1211, 3D 512^3 heat bath 818 -> 1062, 3D 256^3 heat bath 710 -> 858.
 //
 // Lattices below kOneChunkRows chunks run one chunk per thread instead (int8_one_kernel).
