@@ -24,8 +24,9 @@ def assert_same(a, b):
         np.testing.assert_array_equal(x, y)
 
 
+# (the last one's tiles need more shared memory than a kernel has by default)
 @pytest.mark.parametrize("variant,shape", [("msc", (64, 256)), ("int8", (62, 72)),
-                                           ("int8", (64, 64))], ids=str)
+                                           ("int8", (64, 64)), ("int8", (1600, 2488))], ids=str)
 def test_first_sweep_while_another_stream_is_captured(variant, shape):
     import torch
 
