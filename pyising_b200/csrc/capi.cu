@@ -180,15 +180,16 @@ constexpr long long kTemporalInt8 = 6400 * 1024;  // 3500x3584 866 / 839, 4096^2
 constexpr long long kTemporalMsc = 4000 * 4096;   // 5000x4992 2231 / 1876, 6144^2 2388 / 2815
 constexpr long long kTemporalKnobs = 512 * 1024;
 
-static bool use_temporal(const ising_sim* h)
+static bool use_temporal(const ising_sim* h, int64_t every)
 {
     if (h->schedule == ISING_SCHEDULE_TEMPORAL) return temporal_ok(h);
     if (h->schedule != ISING_SCHEDULE_AUTO) return false;
     const long long sites = h->rows * (long long)h->lh;
     if (h->variant == ISING_VARIANT_MSC)
-        return h->msc_kernel == 0 && h->msc_waves == 1 && sites <= kTemporalMsc && temporal_pays(h);
+        return h->msc_kernel == 0 && h->msc_waves == 1 && sites <= kTemporalMsc &&
+               temporal_pays(h, every);
     return sites <= (h->band == 0 && h->vw == 16 ? kTemporalInt8 : kTemporalKnobs) &&
-           temporal_pays(h);
+           temporal_pays(h, every);
 }
 
 // The captured chunk of G sweeps of this handle: 2G half-sweeps with counters relative to the
@@ -705,7 +706,7 @@ int ising_sweep(ising_sim* h, uint64_t t0, int64_t n_sweeps, int64_t measure_eve
     }
     // The tiles need their second pair of arrays.  A stream that is being captured cannot allocate
     // it for later use, and without memory for it the automatic schedule does without the tiles.
-    bool tiles = use_temporal(h);
+    bool tiles = use_temporal(h, n_meas > 0 ? measure_every : 0);
     if (tiles && !(h->tb_scratch[0] && h->tb_scratch[1])) {
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         TRY_CUDA(cudaStreamIsCapturing(h->stream, &capture));

@@ -74,7 +74,8 @@ int half_sweep(ising_sim* h, int color, u32 t, unsigned long long* meas,
 void clear_graphs(ising_sim* h);
 int observe(ising_sim* h, unsigned long long* acc);
 bool temporal_ok(const ising_sim* h);    // the rows fit the temporal schedule's tiles
-bool temporal_pays(const ising_sim* h);  // and tiles are faster than single half-sweeps
+// ... and tiles are faster than single half-sweeps, for sweeps measured each `every` of them (0: none)
+bool temporal_pays(const ising_sim* h, int64_t every);
 // Stream-ordered device memory from the per-device pool that single-lattice handles share.
 cudaError_t pool_alloc(int device, void** p, size_t bytes, cudaStream_t st);
 // The temporal schedule's second pair of colour arrays (allocated once, outside any capture).

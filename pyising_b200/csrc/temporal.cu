@@ -332,9 +332,9 @@ bool temporal_ok(const ising_sim* h)
     return h->ndim == 2 && tile_shape(tile_rows(h)).depth > 0;
 }
 
-bool temporal_pays(const ising_sim* h)
+bool temporal_pays(const ising_sim* h, int64_t every)
 {
-    return h->ndim == 2 && tiles_pay(tile_rows(h));
+    return h->ndim == 2 && tiles_pay(tile_rows(h), every);
 }
 
 template <class Kernel, class... Args>

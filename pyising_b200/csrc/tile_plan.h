@@ -51,10 +51,10 @@ inline TileShape tile_shape(const TileRows& r)
 // nearly as many rows as it keeps.
 constexpr double kTileChunkUs = 2.2e-3, kTileWordUs = 3.35e-3;
 
-inline double tile_half_us(const TileRows& r, const TileShape& s)
+inline double tile_half_us(const TileRows& r, const TileShape& s, double depth)
 {
     const double row_us = (r.msc ? kTileWordUs : kTileChunkUs) * r.units;
-    return (r.msc ? 0.5 : 0.4) + kLaunchUs / s.depth + row_us * (s.band + s.depth - 1);
+    return (r.msc ? 0.5 : 0.4) + kLaunchUs / depth + row_us * (s.band + depth - 1);
 }
 
 // A half-sweep of its own, spread over all SMs.  int8: one chunk per thread.  msc: word ranges up to
@@ -70,18 +70,6 @@ inline double single_half_us(const TileRows& r)
     return (units / rows / 256 > r.sms ? 2.35 : 1.15) + 1.07 * rows;
 }
 
-// Whether tiles beat single half-sweeps.  Measured, flips/ns, tiles / single half-sweeps (and the
-// two times of the model): int8 1024^2 391 / 300 (1.35, 1.94), 64x1024 34 / 26 (1.00, 1.48), 512x4096
-// 451 / 431 (2.42, 2.42), 64x4096 77 / 91 (1.86, 1.57), 64x16384 102 / 265 (5.24, 1.94), 1024x8192
-// 713 / 789 (5.80, 5.35); msc 1152^2 571 / 239 (1.06, 2.66), 4096^2 2116 / 1861 (4.05, 4.49), 6000x5248
-// 2282 / 2364 (6.74, 6.63), 64x8192 169 / 99 (1.69, 2.59), 64x65536 285 / 724 (7.69, 2.90), 128x32768
-// 523 / 731 (4.26, 2.90).
-inline bool tiles_pay(const TileRows& r)
-{
-    const TileShape s = tile_shape(r);
-    return s.depth > 0 && tile_half_us(r, s) <= single_half_us(r);
-}
-
 // A run of `halves` half-sweeps in an even number of launches of about the same depth, at most
 // `depth` each.
 struct TileCuts {
@@ -95,5 +83,29 @@ struct TileCuts {
     }
     int64_t depth(int64_t i) const { return base + (i < longer); }
 };
+
+// Whether tiles beat single half-sweeps.  Measured, flips/ns, tiles / single half-sweeps (and the
+// two times of the model): int8 1024^2 391 / 300 (1.35, 1.94), 64x1024 34 / 26 (1.00, 1.48), 512x4096
+// 451 / 431 (2.42, 2.42), 64x4096 77 / 91 (1.86, 1.57), 64x16384 102 / 265 (5.24, 1.94), 1024x8192
+// 713 / 789 (5.80, 5.35); msc 1152^2 571 / 239 (1.06, 2.66), 4096^2 2116 / 1861 (4.05, 4.49), 6000x5248
+// 2282 / 2364 (6.74, 6.63), 64x8192 169 / 99 (1.69, 2.59), 64x65536 285 / 724 (7.69, 2.90), 128x32768
+// 523 / 731 (4.26, 2.90).
+//
+// Measured every `every` sweeps, a run on tiles is cut at each measurement, and single half-sweeps are
+// replayed as a graph per measurement, whose last kernel, which advances its counters, and next start
+// cost about 4 us more (us per sweep, tiles / graphs: int8 256x8192 measured every sweep 7.4 / 9.5, msc
+// 64x32768 every two 7.2 / 8.4).
+constexpr double kMeasuredGraphUs = 4.0;
+
+inline bool tiles_pay(const TileRows& r, int64_t every)
+{
+    const TileShape s = tile_shape(r);
+    if (s.depth <= 0) return false;
+    if (every <= 0) return tile_half_us(r, s, s.depth) <= single_half_us(r);
+    const TileCuts cuts(2 * every, s.depth);
+    const double halves = 2.0 * every;
+    return halves * tile_half_us(r, s, halves / cuts.launches) <=
+           halves * single_half_us(r) + kMeasuredGraphUs;
+}
 
 }  // namespace ising

@@ -33,15 +33,16 @@ extern "C" int band(long long rows, int ly, int cpr, int sms)
     return ising::int8_default_band(rows, ly, cpr, sms);
 }
 extern "C" int limit(int ndim, int cpr) { return ising::int8_band_limit(ndim, cpr); }
-extern "C" int plan(int msc, int ly, int units, int row_bytes, int sms, int* shape, double* us)
+extern "C" int plan(int msc, int ly, int units, int row_bytes, int sms, int every, int* shape,
+                    double* us)
 {
     const ising::TileRows r{msc != 0, ly, units, (size_t)row_bytes, sms};
     const ising::TileShape s = ising::tile_shape(r);
     shape[0] = s.band;
     shape[1] = s.depth;
-    us[0] = s.depth > 0 ? ising::tile_half_us(r, s) : 0.0;
+    us[0] = s.depth > 0 ? ising::tile_half_us(r, s, s.depth) : 0.0;
     us[1] = ising::single_half_us(r);
-    return ising::tiles_pay(r);
+    return ising::tiles_pay(r, every);
 }
 """
 
@@ -71,12 +72,12 @@ def test_cuts_cover_the_run(plan, sweeps, depth):
         assert launches - 2 < 2 * sweeps / depth  # no more launches than the depth asks for
 
 
-def choose(lib, variant, shape, sms=148):
+def choose(lib, variant, shape, sms=148, every=0):
     ly, lx = shape
     units = lx // 128 if variant == "msc" else -(-lx // 32)
     row_bytes = units * (8 if variant == "msc" else 16)
     out, us = (ctypes.c_int * 2)(), (ctypes.c_double * 2)()
-    pays = lib.plan(int(variant == "msc"), ly, units, row_bytes, sms, out, us)
+    pays = lib.plan(int(variant == "msc"), ly, units, row_bytes, sms, every, out, us)
     band, depth = out
     assert band * sms >= ly and band >= 2
     assert 0 <= depth <= 16 and 2 * depth <= ly
@@ -104,6 +105,17 @@ def choose(lib, variant, shape, sms=148):
 def test_tiles_where_they_are_faster(plan, variant, shape, tiles):
     pays, us = choose(plan, variant, shape)
     assert pays == tiles, us
+    if tiles:  # a graph per measurement costs single half-sweeps more
+        for every in (1, 2, 10, 1000):
+            assert choose(plan, variant, shape, every=every)[0]
+
+
+@pytest.mark.parametrize("variant,shape,every,tiles", [
+    ("int8", (256, 8192), 1, True), ("int8", (256, 8192), 10, False), ("int8", (64, 4096), 1, True),
+    ("int8", (256, 8192), 10**9, False), ("int8", (16, 4096), 2, True), ("msc", (64, 65536), 2, False),
+    ("msc", (128, 32768), 10, False), ("int8", (16, 32768), 1, False)], ids=str)
+def test_measured_sweeps_take_tiles_where_they_are_faster(plan, variant, shape, every, tiles):
+    assert choose(plan, variant, shape, every=every)[0] == tiles
 
 
 LANES = 148 * 512
